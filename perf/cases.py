@@ -190,8 +190,8 @@ def _worlds(case, seed) -> list:
     if kind == "rigid":
         nc, ng = case["circles"], case["polygons"]
         box = 20.0 * math.sqrt(nc + 2 * ng) + 40.0
-        polys = [(_polygon(rng, int(rng.integers(4, 9)), rng.uniform(12.0, box - 12.0, 2),
-                           rng.uniform(4.0, 10.0)), False) for _ in range(ng)]
+        polys = [(_polygon(rng, 4 + k % 5, rng.uniform(12.0, box - 12.0, 2),
+                           rng.uniform(4.0, 10.0)), False) for k in range(ng)]
         return [_world(rng, [], box=box, sub=case["sub"], iters=1,
                        circles=_circles(rng, nc, box, 2.0, 8.0, False), polygons=polys)]
     if kind == "grains":
@@ -208,18 +208,21 @@ def _worlds(case, seed) -> list:
         body = _grid(case["w"], case["h"])
         at = ([(50.0 + pitch * (k % side), 50.0 + pitch * (k // side)) for k in range(n)]
               if case["packed"] else rng.uniform(0.0, box - size, (n, 2)))
-        polys = [(_polygon(rng, int(rng.integers(4, 9)), rng.uniform(50.0, box - 50.0, 2),
+        polys = [(_polygon(rng, 4 + k % 5, rng.uniform(50.0, box - 50.0, 2),
                            rng.uniform(10.0, 50.0)), case["packed"])
-                 for _ in range(case["polygons"])]
+                 for k in range(case["polygons"])]
         return [_world(rng, [_jittered(rng, body, o) for o in at], box=box, sub=case["sub"],
                        iters=case["iters"], fast=case["fast"], collide=ALL, speed=0.5,
                        circles=_circles(rng, case["circles"], box, 5.0, 30.0, case["packed"]),
                        polygons=polys)]
-    sizes = np.exp(rng.uniform(np.log(case["lo"]), np.log(case["hi"]), case["worlds"])).astype(int)
+    # particle counts spread evenly over their logarithm, in a fixed shuffled order
+    k = case["worlds"]
+    sizes = np.exp(np.linspace(np.log(case["lo"]), np.log(case["hi"]), k + 2)[1:-1]).astype(int)
+    sizes = sizes[np.random.default_rng(k).permutation(k)]
     if kind == "rings":  # 1-8 rings of equal size a world
         out = []
-        for n in sizes:
-            k = max(1, min(int(rng.integers(1, 9)), int(n) // 4))
+        for i, n in enumerate(sizes):
+            k = 1 + i % 8
             bodies, stiff = [], []
             for _ in range(k):
                 r = rng.uniform(5.0, 20.0)
