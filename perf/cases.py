@@ -81,7 +81,7 @@ def draw(rng) -> dict:
         return {"kind": kind, "ropes": _log_int(rng, 1, 300), "length": _log_int(rng, 4, 700),
                 "sub": rng.choice([1, 3, 4, 8]), "iters": rng.choice([1, 2, 4])}
     if kind == "rigid":
-        return {"kind": kind, "circles": _log_int(rng, 2, 120), "polygons": _log_int(rng, 1, 40),
+        return {"kind": kind, "circles": _log_int(rng, 2, 40), "polygons": _log_int(rng, 1, 40),
                 "sub": rng.choice([1, 2, 5, 8])}
     if kind == "grains":
         return {"kind": kind, "n": _log_int(rng, 50, 200000), "sub": rng.choice([1, 2, 4, 7])}
