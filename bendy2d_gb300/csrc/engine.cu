@@ -670,7 +670,7 @@ int Engine::rebuild_lists() {
     if (rigid) {
       const uint64_t ng = im.polys.size(), nc = im.cpos.size(), nv = im.vpos.size();
       // same expression as rigid_smem_bytes() in kernels.cuh
-      const uint64_t need = 48 * ng + 28 * nc + 12 * im.clab.size() + 24 * nv +
+      const uint64_t need = 48 * ng + 32 * nc + 12 * im.clab.size() + 24 * nv +
                             12 * im.plab.size() + 8 * im.stage_off.size() + 272;
       if (need <= kRigidSmemCap) rigid_smem = std::max<uint64_t>(rigid_smem, need);
     }
