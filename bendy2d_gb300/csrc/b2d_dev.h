@@ -26,16 +26,12 @@ enum : uint32_t { COLLIDE_PP = 1u, COLLIDE_PC = 2u, COLLIDE_PPOLY = 4u };
 // count kernel for this world.
 constexpr uint32_t GRID_IN_LINKS = 8u;
 
-// Schedule op encoding: link ops carry the body-local link index; bounds +
-// integrate ops carry the body-local particle index with this bit set.
+// Schedule op ids on the host: a body-local link index, or a body-local
+// particle index with this bit set (bounds + integrate).
 constexpr uint32_t OP_INTEG = 0x80000000u;
+// Second word of a link op whose first word is the link index (bodies of more
+// than 65,535 particles, whose endpoints do not fit one word).
 constexpr uint32_t OP_WIDE = 0xFFFFFFFFu;
-// Whole-update schedules only: a padding entry {0, OP_NOP} that does
-// nothing.  Within a level the link solves come first, padded to a whole
-// number of warps, then the bounds+integrate ops, so that no warp runs both
-// code paths (the ops of a level are independent, so their order within the
-// level cannot change any result).
-constexpr uint32_t OP_NOP = 0xFFFFFFFEu;
 
 // A body is a set of solver particles run by one executor unit: a union of
 // whole link-connected components, so no link crosses two bodies.
@@ -45,8 +41,12 @@ struct DBody {
   uint32_t sched;        // schedule id (group executors), else unused
   uint32_t local;        // 1: link endpoints are body-local; 0: world indices
   uint32_t first;        // bidx[i0 + i] == first + i for every i, else NO_FIRST
-  uint32_t pad;
+  uint32_t flags;        // BODY_*
 };
+// Every link's stiffness is exactly 1: the executors keep no stiffness.
+// Every rest length is below 2^100 in magnitude: the fused-arithmetic link
+// solve (kernels.cuh, link_solve_fused) may run.
+enum : uint32_t { BODY_UNIT = 1u, BODY_RANGE = 2u };
 constexpr uint32_t NO_FIRST = 0xFFFFFFFFu;
 
 struct DPoly {
@@ -58,18 +58,24 @@ struct DPoly {
 // A level schedule is stored as a stream of self-describing chunks of at most
 // SCHED_CHUNK_WORDS 32-bit words, each 16-byte aligned so that one bulk copy
 // (TMA, cp.async.bulk) moves it into shared memory:
-//   word 0            nseg
-//   words 1..nseg     end of each segment, counted in ops
+//   word 0            rounds in the chunk
+//   words 1..         the end of each round, counted in the chunk's ops, and
+//                     the last one twice more, so that an executor can load
+//                     two rounds ahead without a test.  Link-pass schedules:
+//                     the end; whole-update schedules: (end of the round's
+//                     link ops) | (end of the round) << 16
 //   (pad to an even word)
-//   then two words per op:
+//   then two words per op, a round's link ops first:
 //     link op    {a | b << 16, link index}   (body-local endpoints; bodies
 //                                             of up to 65535 particles)
 //                {link index, OP_WIDE}       (larger bodies)
-//     integrate  {particle, OP_INTEG}
-//     padding    {0, OP_NOP}                 (whole-update schedules)
-// A segment is a whole level or a piece of one; a group barrier follows
-// every segment.
+//     integrate  {p | p << 16, 0}            (up to 65535 particles)
+//                {p, 0}                      (larger bodies)
+// A round is a whole level, or a piece of one (of at most DSched::tl link ops
+// in schedules for the shared-memory executor); a group barrier follows it.
 constexpr uint32_t SCHED_CHUNK_WORDS = 4096;
+// words before the ops of a chunk of n rounds
+constexpr uint32_t sched_head_words(uint32_t n) { return (n + 4u) & ~1u; }
 // shared bytes after each executor group's schedule area: two mbarriers and
 // two flag words
 constexpr uint32_t GROUP_TAIL_BYTES = 32;
@@ -77,9 +83,8 @@ struct DSched {
   uint32_t chunk0, nchunks;  // chunk_off / chunk_len entries
   uint32_t nlvl, nops;
   uint32_t off, words;       // the chunks are contiguous: stream[off, off + words)
-  uint32_t len0;             // words of the first chunk
-  uint32_t maxw;             // most ops in one segment
-  uint32_t nop_pad;          // 1: the schedule holds OP_NOP padding entries
+  uint32_t tl, ti;           // threads that run link ops and integrate ops (shared-memory
+                             // executor; 0 in schedules for the other executors)
 };
 
 // 1 / c when c is a positive normal power of two (then x / c == x * (1/c)

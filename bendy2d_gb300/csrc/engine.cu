@@ -91,9 +91,10 @@ Engine::Engine(cudaStream_t stream) : stream_(stream) {
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
     for (auto fn : {k_exec_large<true, true>, k_exec_large<false, true>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    for (auto fn : {k_exec_groups<true, true, false>, k_exec_groups<false, true, false>,
-                    k_exec_groups<true, false, false>, k_exec_groups<false, false, false>,
-                    k_exec_groups<true, true, true>, k_exec_groups<false, true, true>})
+    for (auto fn : {k_exec_groups<true, true, false, false>, k_exec_groups<false, true, false, false>,
+                    k_exec_groups<true, true, false, true>, k_exec_groups<false, true, false, true>,
+                    k_exec_groups<true, true, true, false>, k_exec_groups<false, true, true, false>,
+                    k_exec_groups<true, false, false, false>, k_exec_groups<false, false, false, false>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
   }
   tune_.res_max = std::min<uint32_t>(tune_.res_max, (uint32_t)std::max(g_smem_optin, 48 * 1024));
@@ -730,9 +731,14 @@ int Engine::rebuild_lists() {
       c.fill = std::max(c.fill, std::min(room, want));
     }
     const uint32_t per_group = c.region + (c.res ? c.res : 2 * c.fill) + GROUP_TAIL_BYTES;
+    // more bodies than SMs: several share one, and warps without an op in a
+    // round leave their issue slots to the others
+    c.skip = c.items.size() > (size_t)std::max(g_num_sms, 1);
+    // several small groups a CTA, unless each body can have an SM to itself
     uint32_t G = c.T == 32 ? tune_.warp_groups : std::max<uint32_t>(1, 256 / c.T);
     if (c.T != 32) G = std::min<uint32_t>(G, std::min<uint32_t>(tune_.max_groups, 15));
-    G = std::max<uint32_t>(G, 1);
+    G = c.skip ? std::max<uint32_t>(G, 1) : 1;
+    G = std::min<uint32_t>(G, std::max<uint32_t>(1, GROUP_THREADS_MAX / c.T));
     c.G = std::max<uint32_t>(1, std::min<uint32_t>(G, (uint32_t)g_smem_optin / per_group));
   }
   if (!plain_) build_packs(sfull_all, true, packs_full_, serial_full_, true);
@@ -917,9 +923,10 @@ int Engine::launch_all(bool profiling) {
     const bool pdl = !profiling && !c.full && c.res && st == stream_;
     void (*k)(const DWorld*, DScheds, const uint2*, uint32_t, uint32_t, uint32_t, uint32_t,
               uint32_t, uint32_t, uint32_t, uint32_t*, uint2*, DSlots) =
-        c.res ? (c.full ? k_exec_groups<true, true, true> : k_exec_groups<false, true, true>)
-        : c.full ? (c.smem ? k_exec_groups<true, true, false> : k_exec_groups<true, false, false>)
-                 : (c.smem ? k_exec_groups<false, true, false> : k_exec_groups<false, false, false>);
+        c.res ? (c.full ? k_exec_groups<true, true, true, false> : k_exec_groups<false, true, true, false>)
+        : !c.smem ? (c.full ? k_exec_groups<true, false, false, false> : k_exec_groups<false, false, false, false>)
+        : c.skip ? (c.full ? k_exec_groups<true, true, false, true> : k_exec_groups<false, true, false, true>)
+                 : (c.full ? k_exec_groups<true, true, false, false> : k_exec_groups<false, true, false, false>);
     lk(launch_k(k, grid, block, sm, st, pdl, W, SC, L, n, c.T, c.G, rg, sb, cur, sub, GR.count,
                 GR.pbr, GS));
   };

@@ -62,11 +62,11 @@ struct SchedRegistry {
   std::vector<DSched> scheds;
   std::vector<uint32_t> chunk_off, chunk_len, stream;
   size_t uploaded_scheds = 0, uploaded_chunks = 0, uploaded_stream = 0;
-  // wide: the schedule is for the large-body executor, which runs levels
-  // wider than a group (several ops per thread): whole-update schedules are
-  // grouped by op kind there whatever their width
+  // group: for the shared-memory executor, whose rounds hold at most tl link
+  // ops (tl and ti follow from the level widths and t); otherwise a round is
+  // a whole level (or what of it fits a chunk)
   uint32_t get(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I, bool full,
-               bool wide = false);
+               bool group, const PlanTuning& t);
 };
 
 struct GroupBody {
@@ -132,6 +132,7 @@ struct LaunchClass {
   uint32_t fill;   // streamed: bytes per fill buffer (two per group)
   uint32_t words;  // largest member schedule, in words
   bool smem, full;
+  bool skip = false;  // more bodies than SMs: idle warps skip a round's work
   uint32_t large_c = 0, log2per = 0;  // large-body executor class (large_c CTAs per body)
   std::vector<uint2> items;
   size_t dev_off = 0;  // offset (in uint2) into the device list buffer

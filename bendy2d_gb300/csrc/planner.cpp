@@ -50,12 +50,17 @@ bool PlanTuning::set(const std::string& k, double v) {
 }
 
 uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I,
-                            bool full, bool wide) {
+                            bool full, bool group, const PlanTuning& t) {
   std::string key;
-  key.resize(20 + (size_t)nl * 8);
-  const uint32_t hdr[5] = {np, nl, S, I, (full ? 1u : 0u) | (full && wide ? 2u : 0u)};
-  std::memcpy(&key[0], hdr, 20);
-  if (nl) std::memcpy(&key[20], links, (size_t)nl * 8);
+  uint32_t hdr[8] = {np, nl, S, I, (full ? 1u : 0u) | (group ? 2u : 0u), 0u, 0u, 0u};
+  if (group) {
+    hdr[5] = t.t_min;
+    hdr[6] = t.t_max;
+    std::memcpy(&hdr[7], &t.width_per_thread, 4);
+  }
+  key.resize(sizeof(hdr) + (size_t)nl * 8);
+  std::memcpy(&key[0], hdr, sizeof(hdr));
+  if (nl) std::memcpy(&key[sizeof(hdr)], links, (size_t)nl * 8);
   auto it = index.find(key);
   if (it != index.end()) return it->second;
 
@@ -96,73 +101,58 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
     std::vector<uint32_t> fill(start.begin(), start.end());
     for (size_t i = 0; i < total; ++i) sorted[fill[lvl_of[i]]++] = op_of[i];
   }
-  // Whole-update schedules whose levels fit one op per thread of a group of
-  // up to 512: within each level the link solves first, then the
-  // bounds+integrate ops, the links padded with OP_NOP entries to a whole
-  // number of warps (a level's ops are independent, so this order gives the
-  // same results).  A warp then runs one kind only (configuration 1 in
-  // reference order: 378 of 413 levels had a warp running both).  Padding
-  // stays within the power of two above the widest level, so a group that
-  // ran every level with one op per thread still does.  Wider schedules
-  // (fast order: levels of up to ~930 ops, several per thread, and hardly
-  // any mixed warps) keep their order.
-  constexpr uint32_t NOP_ID = 0xFFFFFFFFu;
-  bool padded = false;
-  uint32_t maxw0 = 0;
-  for (uint32_t l = 1; l <= maxl; ++l) maxw0 = std::max(maxw0, start[l + 1] - start[l]);
-  uint32_t cap = 1;
-  while (cap < maxw0) cap <<= 1;
-  if (full && (cap <= 512u || wide)) {
-    std::vector<uint32_t> out, nstart(maxl + 2, 0);
-    out.reserve(total + 32 * (size_t)maxl);
-    for (uint32_t l = 1; l <= maxl; ++l) {
-      nstart[l] = (uint32_t)out.size();
-      const uint32_t b = start[l], e = start[l + 1];
-      uint32_t nlink = 0;
-      for (uint32_t i = b; i < e; ++i)
-        if (!(sorted[i] & OP_INTEG)) {
-          out.push_back(sorted[i]);
-          ++nlink;
-        }
-      const uint32_t ninteg = (e - b) - nlink;
-      const uint32_t pad = (32u - nlink % 32u) % 32u;
-      if (nlink && ninteg && pad && (wide || nlink + pad + ninteg <= cap)) {
-        out.insert(out.end(), pad, NOP_ID);
-        padded = true;
-      }
-      for (uint32_t i = b; i < e; ++i)
-        if (sorted[i] & OP_INTEG) out.push_back(sorted[i]);
-    }
-    nstart[maxl + 1] = (uint32_t)out.size();
-    sorted.swap(out);
-    start.swap(nstart);
+  // a level's link ops first (its ops are independent, so their order within
+  // the level is free); nlink[l] of them
+  std::vector<uint32_t> nlink(maxl + 2, 0);
+  uint32_t max_link = 0, max_integ = 0;
+  for (uint32_t l = 1; l <= maxl; ++l) {
+    const auto b = sorted.begin() + start[l], e = sorted.begin() + start[l + 1];
+    const auto m = full ? std::stable_partition(b, e, [](uint32_t op) { return !(op & OP_INTEG); }) : e;
+    nlink[l] = (uint32_t)(m - b);
+    max_link = std::max(max_link, nlink[l]);
+    max_integ = std::max(max_integ, (uint32_t)(e - m));
   }
-  for (uint32_t op : sorted) {  // self-check: ops name the body's links/particles
-    if (op == NOP_ID) continue;
+  for (uint32_t op : sorted)  // self-check: ops name the body's links/particles
     if ((op & OP_INTEG) ? (op & ~OP_INTEG) >= np : op >= nl) std::abort();
-  }
-  // cut the level sequence into chunks (a level may span chunks)
   DSched d;
   d.chunk0 = (uint32_t)chunk_off.size();
   d.nlvl = maxl;
   d.nops = (uint32_t)total;
+  d.tl = d.ti = 0;
+  if (group) {
+    // Threads for the link ops: the widest level's, in whole warps, within
+    // the tunables; a wider level takes several rounds.  Threads for the
+    // integrate ops: up to 256 (512 in a body without links, which has
+    // nothing else to run); a wider round takes several turns.
+    if (max_link) {
+      const float avg = maxl ? (float)total / (float)maxl : 1.0f;
+      const uint32_t want = pow2ceil((uint32_t)(avg / t.width_per_thread + 0.999f));
+      d.tl = std::min((max_link + 31u) & ~31u, std::max(want, 32u));
+      d.tl = std::min(std::max(d.tl, t.t_min), t.t_max);
+      d.tl = std::min(std::max((d.tl + 31u) & ~31u, 32u), 512u);
+    }
+    if (max_integ) d.ti = std::min((max_integ + 31u) & ~31u, max_link ? 256u : 512u);
+    if (d.tl + d.ti == 0) d.tl = 32;
+  }
+  // cut the level sequence into chunks of rounds (a level may span chunks)
   const bool narrow = np <= 65535u;
-  std::vector<uint32_t> seg_end, chunk_ops;  // chunk_ops: op ids
+  std::vector<uint32_t> ends, chunk_ops;  // chunk_ops: op ids
   auto flush = [&]() {
-    if (seg_end.empty()) return;
+    if (ends.empty()) return;
     while (stream.size() % 4) stream.push_back(0);
     chunk_off.push_back((uint32_t)stream.size());
     const size_t at = stream.size();
-    stream.push_back((uint32_t)seg_end.size());
-    stream.insert(stream.end(), seg_end.begin(), seg_end.end());
+    stream.push_back((uint32_t)ends.size());
+    stream.insert(stream.end(), ends.begin(), ends.end());
+    stream.insert(stream.end(), 2, full ? (uint32_t)chunk_ops.size() * 0x10001u
+                                        : (uint32_t)chunk_ops.size());
     if ((stream.size() - at) % 2) stream.push_back(0);
+    if (stream.size() - at != sched_head_words((uint32_t)ends.size())) std::abort();
     for (uint32_t op : chunk_ops) {
-      if (op == NOP_ID) {
+      if (op & OP_INTEG) {
+        const uint32_t p = op & ~OP_INTEG;
+        stream.push_back(narrow ? p * 0x10001u : p);
         stream.push_back(0);
-        stream.push_back(OP_NOP);
-      } else if (op & OP_INTEG) {
-        stream.push_back(op & ~OP_INTEG);
-        stream.push_back(OP_INTEG);
       } else if (narrow) {
         stream.push_back(links[op].x | (links[op].y << 16));
         stream.push_back(op);
@@ -174,35 +164,42 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
     while ((stream.size() - at) % 4) stream.push_back(0);
     chunk_len.push_back((uint32_t)(stream.size() - at));
     if (chunk_len.back() > SCHED_CHUNK_WORDS) std::abort();
-    seg_end.clear();
+    ends.clear();
     chunk_ops.clear();
   };
+  // ops that still fit the open chunk beside one more round
+  auto room = [&]() -> uint32_t {
+    const size_t used = sched_head_words((uint32_t)ends.size() + 1) + 2 * chunk_ops.size() + 3;
+    return used + 2 > SCHED_CHUNK_WORDS ? 0u : (uint32_t)(SCHED_CHUNK_WORDS - used) / 2;
+  };
   for (uint32_t l = 1; l <= maxl; ++l) {
-    uint32_t b = start[l];
-    const uint32_t e = start[l + 1];
-    while (b < e) {
-      // words: 1 (nseg) + segments (+1 for this one) + 1 pad + 2 per op + 3 pad
-      const size_t fixed = 1 + (seg_end.size() + 1) + 1 + 3;
-      const size_t used = fixed + 2 * chunk_ops.size();
-      if (used + 2 > SCHED_CHUNK_WORDS) {
+    uint32_t lk = start[l], in = start[l] + nlink[l];  // next link op, next integrate op
+    const uint32_t le = in, ie = start[l + 1];
+    while (lk < le || in < ie) {
+      uint32_t want_l = le - lk;
+      if (group && d.tl) want_l = std::min(want_l, d.tl);
+      const uint32_t want = want_l + (ie - in);
+      // a round that fits a chunk of its own is not split between two
+      if (room() == 0 || (room() < want && !ends.empty() && group)) {
         flush();
         continue;
       }
-      const size_t room = (SCHED_CHUNK_WORDS - used) / 2;
-      const uint32_t take = (uint32_t)std::min<size_t>(room, e - b);
-      chunk_ops.insert(chunk_ops.end(), sorted.begin() + b, sorted.begin() + b + take);
-      seg_end.push_back((uint32_t)chunk_ops.size());
-      b += take;
+      const uint32_t tl = std::min(want_l, room());
+      const uint32_t ti = std::min(ie - in, room() - tl);
+      chunk_ops.insert(chunk_ops.end(), sorted.begin() + lk, sorted.begin() + lk + tl);
+      const uint32_t lend = (uint32_t)chunk_ops.size();
+      chunk_ops.insert(chunk_ops.end(), sorted.begin() + in, sorted.begin() + in + ti);
+      const uint32_t end = (uint32_t)chunk_ops.size();
+      ends.push_back(full ? (lend | (end << 16)) : end);
+      lk += tl;
+      in += ti;
     }
   }
   flush();
   d.nchunks = (uint32_t)chunk_off.size() - d.chunk0;
-  d.off = d.words = d.len0 = d.maxw = 0;
-  d.nop_pad = padded ? 1u : 0u;
-  for (uint32_t l = 1; l <= maxl; ++l) d.maxw = std::max(d.maxw, start[l + 1] - start[l]);
+  d.off = d.words = 0;
   if (d.nchunks) {
     d.off = chunk_off[d.chunk0];
-    d.len0 = chunk_len[d.chunk0];
     for (uint32_t c = d.chunk0; c + 1 < d.chunk0 + d.nchunks; ++c)  // self-check: contiguous
       if (chunk_off[c] + chunk_len[c] != chunk_off[c + 1]) std::abort();
     d.words = chunk_off.back() + chunk_len.back() - d.off;
@@ -255,6 +252,7 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
       return bad("large-body executor layout");
     if (g.res && (!g.smem || g.res != S.words * 4u)) return bad("resident schedule size");
     if (g.T < 32 || g.T % 32) return bad("group size");
+    if (g.smem && (S.tl + S.ti != g.T || S.tl % 32 || S.tl > 512u || S.ti > 512u || g.T > 768u)) return bad("group threads");
   }
   for (uint32_t b : im.serials)
     if (b >= im.bodies.size() || !im.bodies[b].local) return bad("serial body");
@@ -397,26 +395,54 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
         im.bidx.push_back(p);
       }
     B.np = n;
-    std::vector<uint2> loc;
+    // The links sorted by their level in one pass (links of one level share no
+    // particle, and each particle still meets its links in order, so this is
+    // the same sequence): the links of a schedule round then sit in a few
+    // consecutive runs, and so do the rest lengths that a warp loads together.
+    struct L2 { uint2 e; float rest, stiff; };
+    std::vector<L2> seq;
+    std::vector<uint32_t> level, depth(n, 0);
+    uint32_t maxd = 0;
     for (const Comp* c : cs)
       for (uint32_t k : c->links) {
         const Link& L = w.particle_links[k];
-        loc.push_back(make_uint2(local[L.particle_a], local[L.particle_b]));
-        im.lrest.push_back(L.target_distance);
-        im.lstiff.push_back(L.stiffness);
+        const uint32_t a = local[L.particle_a], b = local[L.particle_b];
+        const uint32_t l = std::max(depth[a], depth[b]);
+        depth[a] = depth[b] = l + 1;
+        maxd = std::max(maxd, l + 1);
+        level.push_back(l);
+        seq.push_back(L2{make_uint2(a, b), L.target_distance, L.stiffness});
       }
+    std::vector<uint32_t> at(maxd + 1, 0);
+    for (uint32_t l : level) ++at[l + 1];
+    for (uint32_t l = 0; l < maxd; ++l) at[l + 1] += at[l];
+    std::vector<uint2> loc(seq.size());
+    im.lrest.resize(B.l0 + seq.size());
+    im.lstiff.resize(B.l0 + seq.size());
+    for (size_t k = 0; k < seq.size(); ++k) {
+      const uint32_t i = at[level[k]]++;
+      loc[i] = seq[k].e;
+      im.lrest[B.l0 + i] = seq[k].rest;
+      im.lstiff[B.l0 + i] = seq[k].stiff;
+    }
     B.nl = (uint32_t)loc.size();
-    const size_t region = align16((full ? 16u : 8u) * (size_t)B.np + 8u * (size_t)B.nl);
-    const bool smem = region <= tune.smem_max && B.np <= 65535u;
-    // whether the large-body executor (below) will run it
-    const bool to_large = !smem && tune.large_max > 0 && B.np > 0 &&
-                          (B.np + (1u << (full ? 13u : 14u)) - 1u) >> (full ? 13u : 14u) <=
-                              tune.large_max;
-    B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, to_large);
+    B.flags = BODY_UNIT | BODY_RANGE;
+    for (uint32_t k = 0; k < B.nl; ++k) {
+      const float r = im.lrest[B.l0 + k];
+      if (im.lstiff[B.l0 + k] != 1.0f) B.flags &= ~BODY_UNIT;
+      if (!(r < 0x1p100f && r > -0x1p100f)) B.flags &= ~BODY_RANGE;
+    }
+    // the executor is chosen by the body's size with stiffness; a body of
+    // unit stiffness takes less
+    const size_t state = (full ? 16u : 8u) * (size_t)B.np;
+    const bool smem = align16(state + 8u * (size_t)B.nl) <= tune.smem_max && B.np <= 65535u;
+    const size_t region = align16(state + (B.flags & BODY_UNIT ? 4u : 8u) * (size_t)B.nl);
+    B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, smem, tune);
     const DSched& S = reg.scheds[B.sched];
     const float avg = S.nlvl ? (float)S.nops / (float)S.nlvl : 1.0f;
     uint32_t T = pow2ceil((uint32_t)(avg / tune.width_per_thread + 0.999f));
     T = std::min(std::max(T, tune.t_min), tune.t_max);
+    if (smem) T = S.tl + S.ti;
     // the whole schedule resident in shared memory when it fits beside the body
     uint32_t res = 0;
     if (smem && tune.resident) {
