@@ -284,21 +284,28 @@ struct Comp {
   std::vector<uint32_t> links;  // world link ids in execution order
 };
 
-uint32_t single_pass_depth(const WorldHost& w, const Comp& c, std::vector<uint32_t>& last) {
-  uint32_t depth = 0;
-  for (uint32_t k : c.links) {
-    const uint32_t a = (uint32_t)w.particle_links[k].particle_a;
-    const uint32_t b = (uint32_t)w.particle_links[k].particle_b;
-    const uint32_t l = std::max(last[a], last[b]) + 1;
-    last[a] = l;
-    last[b] = l;
-    depth = std::max(depth, l);
+// Levels of one pass over the component's links, and how many a second pass
+// adds.  (A rope's second pass starts two levels behind its first, a ring's
+// only once the spokes have moved the rim again.)
+struct PassDepth { uint32_t first, more; };
+PassDepth pass_depth(const WorldHost& w, const Comp& c, std::vector<uint32_t>& last) {
+  uint32_t depth[2] = {0, 0};
+  for (int pass = 0; pass < 2; ++pass) {
+    depth[pass] = pass ? depth[0] : 0u;
+    for (uint32_t k : c.links) {
+      const uint32_t a = (uint32_t)w.particle_links[k].particle_a;
+      const uint32_t b = (uint32_t)w.particle_links[k].particle_b;
+      const uint32_t l = std::max(last[a], last[b]) + 1;
+      last[a] = l;
+      last[b] = l;
+      depth[pass] = std::max(depth[pass], l);
+    }
   }
   for (uint32_t k : c.links) {
     last[w.particle_links[k].particle_a] = 0;
     last[w.particle_links[k].particle_b] = 0;
   }
-  return depth;
+  return PassDepth{depth[0], depth[1] - depth[0]};
 }
 }  // namespace
 
@@ -498,9 +505,18 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
       free_parts.push_back(c.parts[0]);
       continue;
     }
-    const uint32_t depth = single_pass_depth(w, c, last);
-    const float width = (float)c.links.size() / (float)std::max(depth, 1u);
-    if (width < tune.serial_width) {
+    // Serial or by levels: a body whose single pass is narrow may still be wide
+    // over the passes its schedule chains, which start behind one another.
+    // Measured on 24 ropes of 200 particles (one pass 1 wide, the 8 x 4 passes
+    // of an update ~29): 1,710 us a pass replayed by one thread each, 79 us by
+    // levels.  Rings of a hub and spokes stay below 3 (the next pass's rim
+    // runs beside this pass's spokes) and run serially.
+    const PassDepth pd = pass_depth(w, c, last);
+    const double passes = full ? (double)P.S * P.I : (double)P.I;
+    const double ops = passes * (double)c.links.size() + (full ? (double)P.S * c.parts.size() : 0.0);
+    const double levels = (double)pd.first + (passes - 1.0) * pd.more + (full ? (double)P.S : 0.0);
+    const double width = (double)c.links.size() / (double)std::max(pd.first, 1u);
+    if (width < tune.serial_width && ops / std::max(levels, 1.0) < 1.5 * tune.serial_width) {
       DBody B{};
       B.i0 = (uint32_t)im.bidx.size();
       B.np = (uint32_t)c.parts.size();
