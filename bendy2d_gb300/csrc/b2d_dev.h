@@ -37,8 +37,10 @@ constexpr uint32_t OP_WIDE = 0xFFFFFFFFu;
 // whole link-connected components, so no link crosses two bodies.
 struct DBody {
   uint32_t i0, np;       // particle list bidx[i0 .. i0+np) (world indices, ascending)
-  uint32_t l0, nl;       // links lab[l0 .. l0+nl) in insertion order
-  uint32_t sched;        // schedule id (group executors), else unused
+  uint32_t l0, nl;       // links lab[l0 .. l0+nl) (serial bodies: lrec) in execution order
+  uint32_t sched;        // schedule id (group executors); serial bodies: links of the first
+                         // half, which runs beside the second half of the pass before it
+                         // a lag (flags >> BODY_LAG_SHIFT) behind (0: the links run in one chain)
   uint32_t local;        // 1: link endpoints are body-local; 0: world indices
   uint32_t first;        // bidx[i0 + i] == first + i for every i, else NO_FIRST
   uint32_t flags;        // BODY_*
@@ -46,7 +48,12 @@ struct DBody {
 // Every link's stiffness is exactly 1: the executors keep no stiffness.
 // Every rest length is below 2^100 in magnitude: the fused-arithmetic link
 // solve (kernels.cuh, link_solve_fused) may run.
-enum : uint32_t { BODY_UNIT = 1u, BODY_RANGE = 2u };
+// A serial executor's body.
+enum : uint32_t { BODY_UNIT = 1u, BODY_RANGE = 2u, BODY_SERIAL = 4u };
+constexpr uint32_t BODY_LAG_SHIFT = 8;
+// Mark on a link endpoint of a serial body in two chains: no later link of
+// the pass moves this particle (it is integrated right after).
+constexpr uint32_t LINK_FINAL = 0x80000000u;
 constexpr uint32_t NO_FIRST = 0xFFFFFFFFu;
 
 struct DPoly {
@@ -124,6 +131,8 @@ struct DWorld {
   uint2* lab;
   float* lrest;
   float* lstiff;
+  uint4* lrec;           // serial bodies' links: {a, b, rest bits, stiffness bits}, endpoints
+                         // body-local with their LINK_FINAL marks
   // circles (src/circle.rs:4-8) and circle links
   float2* cpos; float2* cprev; float2* cacc;
   float* crad; uint32_t* cstatic;

@@ -44,7 +44,6 @@ static constexpr uint64_t kRigidSmemCap = 96 * 1024;
 // 1024-thread CTAs (k_rigid<MODE, 1024>), the others in 256-thread CTAs
 static constexpr uint64_t kRigidWideTests = 4096;
 static constexpr uint32_t kSerialPackBytes = 96 * 1024;  // shared memory per small-body pack
-static constexpr uint32_t kSerialPackThreads = 64;       // bodies per serial pack
 
 // Kernel launch; pdl: programmatic dependent launch — the kernel may start
 // while the previous kernel in the stream finishes (it calls pdl_wait()
@@ -192,6 +191,7 @@ int Engine::fill_world_record(uint32_t slot) {
   W.lab = reinterpret_cast<uint2*>(b + L.o_lab);
   W.lrest = reinterpret_cast<float*>(b + L.o_lrest);
   W.lstiff = reinterpret_cast<float*>(b + L.o_lstiff);
+  W.lrec = reinterpret_cast<uint4*>(b + L.o_lrec);
   W.cpos = reinterpret_cast<float2*>(b + L.o_cpos);
   W.cprev = reinterpret_cast<float2*>(b + L.o_cprev);
   W.cacc = reinterpret_cast<float2*>(b + L.o_cacc);
@@ -496,18 +496,15 @@ int Engine::ensure_grid(size_t nbuckets, size_t np_pp) {
   return OK;
 }
 
-// First-fit decreasing: bodies sorted by size, each into the first pack with
-// room (bytes and threads).  Bodies larger than a pack stay in `rest` for the
-// global-memory serial kernel.
 // Serial packs.  The step time of a batch of chain-like bodies follows its
-// longest chains.  A body whose chain is at least stage_frac (default 2/3)
-// of the longest gets a pack of its own with the links staged too (8 or 16 B
-// per particle plus 16 B per link, up to the shared-memory limit; at most
-// one per SM; allow_large): staging cuts a link from ~333 to ~211 cycles, so
-// shorter chains finish in time without it and leave the SMs' shared memory
-// to the packs of many bodies (positions only, first-fit decreasing, up to
-// kSerialPackBytes and kSerialPackThreads bodies).  What fits neither stays
-// in `rest` for the global-memory serial kernel.
+// longest chains.  A body whose chain is at least stage_frac of the longest
+// gets a pack of its own with the links staged too (8 or 16 B per particle
+// plus 16 B per link, up to the shared-memory limit; at most one per SM;
+// allow_large); the default (1.01) makes none: with the records streamed
+// through a ring the ordinary packs run as fast.  The others go first-fit
+// decreasing into packs of positions only, up to kSerialPackBytes and
+// SERIAL_PACK_BODIES bodies.  What fits neither stays in `rest` for the
+// global-memory serial kernel.
 void Engine::build_packs(std::vector<uint2>& in, bool full, SerialPacks* out,
                          std::vector<uint2>& rest, bool allow_large) {
   const uint32_t per = full ? 16u : 8u;
@@ -535,10 +532,11 @@ void Engine::build_packs(std::vector<uint2>& in, bool full, SerialPacks* out,
       pb += body(it).np;
       lb += body(it).nl;
     }
-    o.max_bytes = std::max(o.max_bytes, pb * per + (staged ? lb * 16u : 0u));
+    o.max_bytes = std::max(o.max_bytes,
+                           pb * per + (staged ? lb * 16u + SERIAL_STAGED_EXTRA : SERIAL_EXTRA));
   };
   for (const uint2& it : in) {
-    if (n_large < max_large && long_chain(it) && bytes_of(it) <= large_cap) {  // longest chains
+    if (n_large < max_large && long_chain(it) && bytes_of(it) + SERIAL_STAGED_EXTRA <= large_cap) {  // longest chains
       emit(out[1], std::vector<uint2>{it}, true);
       ++n_large;
       continue;
@@ -550,7 +548,7 @@ void Engine::build_packs(std::vector<uint2>& in, bool full, SerialPacks* out,
     }
     size_t k = first_open;
     while (k < bins.size() && (used[k] + bytes > kSerialPackBytes ||
-                               bins[k].size() >= kSerialPackThreads))
+                               bins[k].size() >= SERIAL_PACK_BODIES))
       ++k;
     if (k == bins.size()) {
       bins.emplace_back();
@@ -558,7 +556,7 @@ void Engine::build_packs(std::vector<uint2>& in, bool full, SerialPacks* out,
     }
     bins[k].push_back(it);
     used[k] += bytes;
-    while (first_open < bins.size() && bins[first_open].size() >= kSerialPackThreads) ++first_open;
+    while (first_open < bins.size() && bins[first_open].size() >= SERIAL_PACK_BODIES) ++first_open;
   }
   for (const auto& bin : bins) emit(out[0], bin, false);
 }
@@ -957,7 +955,7 @@ int Engine::launch_all(bool profiling) {
       if (wl.pkn) {
         const SerialPacks& P = packs_full_[0];
         timed("plain_exec_serial_smem", [&] {
-          k_exec_serial_smem<true, false><<<wl.pkn, kSerialPackThreads, P.max_bytes, stream_>>>(
+          k_exec_serial_smem<true, false><<<wl.pkn, SERIAL_THREADS, P.max_bytes, stream_>>>(
               W, d_lists_ + P.off_items, d_lists_ + P.off_base, d_lists_ + P.off_packs + wl.pk0,
               wl.pkn, 0, 0);
         });
@@ -987,7 +985,7 @@ int Engine::launch_all(bool profiling) {
     const uint32_t n = (uint32_t)P.packs.size();
     const cudaStream_t st = branch();
     timed(k == 0 ? "exec_serial_smem_full" : "exec_serial_staged_full", [&] {
-      if (k == 0) k_exec_serial_smem<true, false><<<n, kSerialPackThreads, P.max_bytes, st>>>(
+      if (k == 0) k_exec_serial_smem<true, false><<<n, SERIAL_THREADS, P.max_bytes, st>>>(
           W, d_lists_ + P.off_items, d_lists_ + P.off_base, d_lists_ + P.off_packs, n, 0, 0);
       else k_exec_serial_smem<true, true><<<n, 32, P.max_bytes, st>>>(
           W, d_lists_ + P.off_items, d_lists_ + P.off_base, d_lists_ + P.off_packs, n, 0, 0);
@@ -1035,7 +1033,7 @@ int Engine::launch_all(bool profiling) {
       const uint32_t n = (uint32_t)P.packs.size();
       const cudaStream_t st = branch();
       timed(k == 0 ? "exec_serial_smem_links" : "exec_serial_staged_links", [&] {
-        if (k == 0) k_exec_serial_smem<false, false><<<n, kSerialPackThreads, P.max_bytes, st>>>(
+        if (k == 0) k_exec_serial_smem<false, false><<<n, SERIAL_THREADS, P.max_bytes, st>>>(
             W, d_lists_ + P.off_items, d_lists_ + P.off_base, d_lists_ + P.off_packs, n, cur, s);
         else k_exec_serial_smem<false, true><<<n, 32, P.max_bytes, st>>>(
             W, d_lists_ + P.off_items, d_lists_ + P.off_base, d_lists_ + P.off_packs, n, cur, s);

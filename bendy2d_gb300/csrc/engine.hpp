@@ -98,6 +98,7 @@ struct WorldImage {
   std::vector<DBody> bodies;
   std::vector<uint2> lab;
   std::vector<float> lrest, lstiff;
+  std::vector<uint4> lrec;  // serial bodies' links
   std::vector<float> crad;
   std::vector<uint32_t> cstatic;
   std::vector<uint2> clab;
@@ -121,7 +122,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
 struct BlockLayout {
   size_t state_bytes = 0, total = 0;
   size_t o_pos, o_prev, o_cpos, o_cprev, o_cacc, o_vpos, o_vprev, o_vacc, o_pcenter;
-  size_t o_pos1, o_bidx, o_bodies, o_lab, o_lrest, o_lstiff, o_crad, o_cstatic, o_clab,
+  size_t o_pos1, o_bidx, o_bodies, o_lab, o_lrest, o_lstiff, o_lrec, o_crad, o_cstatic, o_clab,
       o_clrest, o_polys, o_paabb, o_plab, o_plrest, o_stage, o_stage_pr;
 };
 BlockLayout layout_of(const WorldImage& im);

@@ -224,8 +224,9 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
   if (im.bodies.size() != P.nb) return bad("body count");
   for (const DBody& B : im.bodies) {
     if ((size_t)B.i0 + B.np > im.bidx.size()) return bad("body particle range");
-    if ((size_t)B.l0 + B.nl > im.lab.size() || im.lab.size() != im.lrest.size() ||
-        im.lab.size() != im.lstiff.size())
+    const bool serial = (B.flags & BODY_SERIAL) != 0u;
+    if ((size_t)B.l0 + B.nl > (serial ? im.lrec.size() : im.lab.size()) ||
+        im.lab.size() != im.lrest.size() || im.lab.size() != im.lstiff.size())
       return bad("body link range");
     for (uint32_t i = 0; i < B.np; ++i)
       if (im.bidx[B.i0 + i] >= P.np) return bad("body particle index");
@@ -234,7 +235,9 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
       return bad("body first particle");
     const uint32_t lim = B.local ? B.np : P.np;
     for (uint32_t k = 0; k < B.nl; ++k) {
-      const uint2 e = im.lab[B.l0 + k];
+      const uint2 e = serial ? make_uint2(im.lrec[B.l0 + k].x & ~LINK_FINAL,
+                                          im.lrec[B.l0 + k].y & ~LINK_FINAL)
+                             : im.lab[B.l0 + k];
       if (e.x >= lim || e.y >= lim || e.x == e.y) return bad("link endpoint");
     }
   }
@@ -254,8 +257,13 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
     if (g.T < 32 || g.T % 32) return bad("group size");
     if (g.smem && (S.tl + S.ti != g.T || S.tl % 32 || S.tl > 512u || S.ti > 512u || g.T > 768u)) return bad("group threads");
   }
-  for (uint32_t b : im.serials)
-    if (b >= im.bodies.size() || !im.bodies[b].local) return bad("serial body");
+  for (uint32_t b : im.serials) {
+    if (b >= im.bodies.size() || !im.bodies[b].local || !(im.bodies[b].flags & BODY_SERIAL))
+      return bad("serial body");
+    const DBody& B = im.bodies[b];
+    if (B.sched && (B.sched >= B.nl || B.nl - B.sched < (B.flags >> BODY_LAG_SHIFT)))
+      return bad("serial body halves");
+  }
   if (im.cpos.size() != P.nc || im.crad.size() != P.nc) return bad("circle arrays");
   for (const uint2& e : im.clab)
     if (e.x >= P.nc || e.y >= P.nc) return bad("circle link");
@@ -285,13 +293,15 @@ struct Comp {
 };
 
 // Levels of one pass over the component's links, and how many a second pass
-// adds.  (A rope's second pass starts two levels behind its first, a ring's
-// only once the spokes have moved the rim again.)
+// adds (0 where the first pass alone is `enough` wide).  A rope's second pass
+// starts two levels behind its first, a ring's only once the spokes have moved
+// the rim again.
 struct PassDepth { uint32_t first, more; };
-PassDepth pass_depth(const WorldHost& w, const Comp& c, std::vector<uint32_t>& last) {
+PassDepth pass_depth(const WorldHost& w, const Comp& c, float enough, std::vector<uint32_t>& last) {
   uint32_t depth[2] = {0, 0};
   for (int pass = 0; pass < 2; ++pass) {
-    depth[pass] = pass ? depth[0] : 0u;
+    depth[pass] = depth[0];
+    if (pass && (float)c.links.size() / (float)std::max(depth[0], 1u) >= enough) break;
     for (uint32_t k : c.links) {
       const uint32_t a = (uint32_t)w.particle_links[k].particle_a;
       const uint32_t b = (uint32_t)w.particle_links[k].particle_b;
@@ -306,6 +316,42 @@ PassDepth pass_depth(const WorldHost& w, const Comp& c, std::vector<uint32_t>& l
     last[w.particle_links[k].particle_b] = 0;
   }
   return PassDepth{depth[0], depth[1] - depth[0]};
+}
+// Whether the second half of a serial body's links can run beside the first
+// half of the next pass, a lag behind it: step j solves link j of the second
+// half and link j - lag of the next first half; a particle is integrated a step
+// after the link that moves it last.  So every particle of first-half link i
+// must have been moved for the last time in the pass by step i + lag - 2, and
+// every particle must be moved by some link of the second half.  A link integrates one particle; only the last, which
+// moves both of its particles last, has a step more for the other.  Taken when
+// the lag is at most a quarter of the half: then B.sched is the first half's
+// length, the lag is in B.flags, and the last link of the pass that moves a
+// particle marks it (LINK_FINAL).
+void split_chain(DBody& B, uint4* ab) {
+  B.sched = 0;
+  const uint32_t m = B.nl / 2, nb = B.nl - m;
+  if (m < 8) return;
+  constexpr uint32_t NONE = 0xFFFFFFFFu;
+  std::vector<uint32_t> last(B.np, NONE);  // the particle's last link in the second half
+  for (uint32_t j = 0; j < nb; ++j) last[ab[m + j].x] = last[ab[m + j].y] = j;
+  for (uint32_t l : last)
+    if (l == NONE) return;
+  for (uint32_t j = 0; j + 1 < nb; ++j)
+    if (last[ab[m + j].x] == j && last[ab[m + j].y] == j) return;
+  const uint32_t other = ab[B.nl - 1].y;  // integrated a step after the last link
+  uint32_t lag = 1;
+  for (uint32_t i = 0; i < m; ++i) {
+    uint32_t l = std::max(last[ab[i].x], last[ab[i].y]) + 2u;
+    if (ab[i].x == other || ab[i].y == other) l = nb + 2u;
+    if (l > i) lag = std::max(lag, l - i);
+    if (lag > nb / 4) return;
+  }
+  for (uint32_t p = 0; p < B.np; ++p) {
+    uint4& e = ab[m + last[p]];
+    (e.x == p ? e.x : e.y) |= LINK_FINAL;
+  }
+  B.sched = m;
+  B.flags |= lag << BODY_LAG_SHIFT;
 }
 }  // namespace
 
@@ -406,9 +452,12 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // particle, and each particle still meets its links in order, so this is
     // the same sequence): the links of a schedule round then sit in a few
     // consecutive runs, and so do the rest lengths that a warp loads together.
-    struct L2 { uint2 e; float rest, stiff; };
-    std::vector<L2> seq;
-    std::vector<uint32_t> level, depth(n, 0);
+    size_t links = 0;
+    for (const Comp* c : cs) links += c->links.size();
+    struct Item { uint2 e; float rest, stiff; uint32_t level; };
+    std::vector<Item> seq;
+    seq.reserve(links);
+    std::vector<uint32_t> depth(n, 0);
     uint32_t maxd = 0;
     for (const Comp* c : cs)
       for (uint32_t k : c->links) {
@@ -417,20 +466,19 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
         const uint32_t l = std::max(depth[a], depth[b]);
         depth[a] = depth[b] = l + 1;
         maxd = std::max(maxd, l + 1);
-        level.push_back(l);
-        seq.push_back(L2{make_uint2(a, b), L.target_distance, L.stiffness});
+        seq.push_back(Item{make_uint2(a, b), L.target_distance, L.stiffness, l});
       }
     std::vector<uint32_t> at(maxd + 1, 0);
-    for (uint32_t l : level) ++at[l + 1];
+    for (const Item& it : seq) ++at[it.level + 1];
     for (uint32_t l = 0; l < maxd; ++l) at[l + 1] += at[l];
     std::vector<uint2> loc(seq.size());
     im.lrest.resize(B.l0 + seq.size());
     im.lstiff.resize(B.l0 + seq.size());
-    for (size_t k = 0; k < seq.size(); ++k) {
-      const uint32_t i = at[level[k]]++;
-      loc[i] = seq[k].e;
-      im.lrest[B.l0 + i] = seq[k].rest;
-      im.lstiff[B.l0 + i] = seq[k].stiff;
+    for (const Item& it : seq) {
+      const uint32_t i = at[it.level]++;
+      loc[i] = it.e;
+      im.lrest[B.l0 + i] = it.rest;
+      im.lstiff[B.l0 + i] = it.stiff;
     }
     B.nl = (uint32_t)loc.size();
     B.flags = BODY_UNIT | BODY_RANGE;
@@ -511,7 +559,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // of an update ~29): 1,710 us a pass replayed by one thread each, 79 us by
     // levels.  Rings of a hub and spokes stay below 3 (the next pass's rim
     // runs beside this pass's spokes) and run serially.
-    const PassDepth pd = pass_depth(w, c, last);
+    const PassDepth pd = pass_depth(w, c, tune.serial_width, last);
     const double passes = full ? (double)P.S * P.I : (double)P.I;
     const double ops = passes * (double)c.links.size() + (full ? (double)P.S * c.parts.size() : 0.0);
     const double levels = (double)pd.first + (passes - 1.0) * pd.more + (full ? (double)P.S : 0.0);
@@ -520,7 +568,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
       DBody B{};
       B.i0 = (uint32_t)im.bidx.size();
       B.np = (uint32_t)c.parts.size();
-      B.l0 = (uint32_t)im.lab.size();
+      B.l0 = (uint32_t)im.lrec.size();
       B.nl = (uint32_t)c.links.size();
       B.local = 1;  // body-local endpoints: index into the body's particle list
       uint32_t nloc = 0;
@@ -528,12 +576,16 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
         local[p] = nloc++;
         im.bidx.push_back(p);
       }
+      B.flags = BODY_SERIAL | BODY_RANGE;
       for (uint32_t k : c.links) {
         const Link& L = w.particle_links[k];
-        im.lab.push_back(make_uint2(local[L.particle_a], local[L.particle_b]));
-        im.lrest.push_back(L.target_distance);
-        im.lstiff.push_back(L.stiffness);
+        uint32_t rs[2];
+        std::memcpy(&rs[0], &L.target_distance, 4);
+        std::memcpy(&rs[1], &L.stiffness, 4);
+        im.lrec.push_back(make_uint4(local[L.particle_a], local[L.particle_b], rs[0], rs[1]));
+        if (!(L.target_distance < 0x1p100f && L.target_distance > -0x1p100f)) B.flags &= ~BODY_RANGE;
       }
+      split_chain(B, &im.lrec[B.l0]);
       im.serials.push_back((uint32_t)im.bodies.size());
       im.bodies.push_back(B);
       im.stats.serial_bodies++;
@@ -654,6 +706,7 @@ BlockLayout layout_of(const WorldImage& im) {
   L.o_lab = seg(8 * im.lab.size());
   L.o_lrest = seg(4 * im.lrest.size());
   L.o_lstiff = seg(4 * im.lstiff.size());
+  L.o_lrec = seg(16 * im.lrec.size());
   L.o_crad = seg(4 * nc);
   L.o_cstatic = seg(4 * nc);
   L.o_clab = seg(8 * im.clab.size());
@@ -688,6 +741,7 @@ void write_block(const WorldImage& im, const BlockLayout& L, unsigned char* dst)
   put(L.o_lab, im.lab.data(), 8 * im.lab.size());
   put(L.o_lrest, im.lrest.data(), 4 * im.lrest.size());
   put(L.o_lstiff, im.lstiff.data(), 4 * im.lstiff.size());
+  put(L.o_lrec, im.lrec.data(), 16 * im.lrec.size());
   put(L.o_crad, im.crad.data(), 4 * im.crad.size());
   put(L.o_cstatic, im.cstatic.data(), 4 * im.cstatic.size());
   put(L.o_clab, im.clab.data(), 8 * im.clab.size());
