@@ -437,6 +437,9 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
   std::vector<const Comp*> pack;
   uint32_t pack_np = 0, pack_nl = 0;
 
+  struct Item { uint2 e; float rest, stiff; uint32_t level; };
+  std::vector<Item> seq;                // emit_group's, kept between bodies
+  std::vector<uint32_t> depth, at;
   auto emit_group = [&](const std::vector<const Comp*>& cs) {
     DBody B{};
     B.i0 = (uint32_t)im.bidx.size();
@@ -452,40 +455,32 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // particle, and each particle still meets its links in order, so this is
     // the same sequence): the links of a schedule round then sit in a few
     // consecutive runs, and so do the rest lengths that a warp loads together.
-    size_t links = 0;
-    for (const Comp* c : cs) links += c->links.size();
-    struct Item { uint2 e; float rest, stiff; uint32_t level; };
-    std::vector<Item> seq;
-    seq.reserve(links);
-    std::vector<uint32_t> depth(n, 0);
-    uint32_t maxd = 0;
+    seq.clear();
+    depth.assign(n, 0);
+    at.assign(1, 0);
     for (const Comp* c : cs)
       for (uint32_t k : c->links) {
         const Link& L = w.particle_links[k];
         const uint32_t a = local[L.particle_a], b = local[L.particle_b];
-        const uint32_t l = std::max(depth[a], depth[b]);
-        depth[a] = depth[b] = l + 1;
-        maxd = std::max(maxd, l + 1);
-        seq.push_back(Item{make_uint2(a, b), L.target_distance, L.stiffness, l});
+        const uint32_t l = std::max(depth[a], depth[b]) + 1;
+        depth[a] = depth[b] = l;
+        if (l == at.size()) at.push_back(0);
+        ++at[l];
+        seq.push_back(Item{make_uint2(a, b), L.target_distance, L.stiffness, l - 1});
       }
-    std::vector<uint32_t> at(maxd + 1, 0);
-    for (const Item& it : seq) ++at[it.level + 1];
-    for (uint32_t l = 0; l < maxd; ++l) at[l + 1] += at[l];
+    for (size_t l = 1; l < at.size(); ++l) at[l] += at[l - 1];
     std::vector<uint2> loc(seq.size());
     im.lrest.resize(B.l0 + seq.size());
     im.lstiff.resize(B.l0 + seq.size());
+    B.nl = (uint32_t)seq.size();
+    B.flags = BODY_UNIT | BODY_RANGE;
     for (const Item& it : seq) {
       const uint32_t i = at[it.level]++;
       loc[i] = it.e;
       im.lrest[B.l0 + i] = it.rest;
       im.lstiff[B.l0 + i] = it.stiff;
-    }
-    B.nl = (uint32_t)loc.size();
-    B.flags = BODY_UNIT | BODY_RANGE;
-    for (uint32_t k = 0; k < B.nl; ++k) {
-      const float r = im.lrest[B.l0 + k];
-      if (im.lstiff[B.l0 + k] != 1.0f) B.flags &= ~BODY_UNIT;
-      if (!(r < 0x1p100f && r > -0x1p100f)) B.flags &= ~BODY_RANGE;
+      if (it.stiff != 1.0f) B.flags &= ~BODY_UNIT;
+      if (!(it.rest < 0x1p100f && it.rest > -0x1p100f)) B.flags &= ~BODY_RANGE;
     }
     // the executor is chosen by the body's size with stiffness; a body of
     // unit stiffness takes less
