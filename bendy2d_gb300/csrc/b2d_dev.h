@@ -90,9 +90,43 @@ struct DSched {
   uint32_t chunk0, nchunks;  // chunk_off / chunk_len entries
   uint32_t nlvl, nops;
   uint32_t off, words;       // the chunks are contiguous: stream[off, off + words)
-  uint32_t tl, ti;           // threads that run link ops and integrate ops (shared-memory
-                             // executor; 0 in schedules for the other executors)
+  uint32_t tl, ti;           // threads that run link ops and integrate ops (shared-memory and
+                             // flow executors; 0 in schedules for the other executors)
 };
+
+// Flow schedules (large bodies, k_exec_flow): the C CTAs of a cluster each run
+// their own ops of every level, in chunks like the above (DSched::off: C
+// records of FLOW_REC_WORDS words, below), except that
+//   a round's word is   link ops end | round end << 11 | level % 32 << 22
+//                       (the two after the last carry the next round's level)
+//   an op is            {a | b << 16, k | to(a) << 16 | to(b) << 23}
+//                       with k the CTA's own link index; to(x), where the
+//                       particle goes after this op: bit 0 set when its next
+//                       user is another CTA, bits 1-3 that CTA, bits 4-6 one
+//                       less than the levels until it has to be there
+// and one more op {lo | lo << 16, 0} ends each chunk (in no round), so that a
+// chunk without ops has one to read.
+constexpr uint32_t FLOW_REC_WORDS = 16;
+enum : uint32_t {            // words of a CTA's record
+  FR_CHUNK0, FR_NCHUNKS,     // its chunks: chunk_off / chunk_len entries
+  FR_LO, FR_WINDOW,          // body-local ids [lo, lo + window) have a slot here
+  FR_OWN0, FR_OWN1,          // particles it integrates
+  FR_LINKS, FR_NLINKS,       // stream offset: body link of each of its link indices
+  FR_LOAD, FR_NLOAD,         // particles that start here
+  FR_STORE, FR_NSTORE,       // particles that end here
+  FR_EXPECT, FR_NLEVELS,     // per level: particles that have to arrive before it
+};
+// shared bytes beside a flow CTA's state: the cluster's addresses, arrival, progress and fill
+// barriers, the flags, the chunk count of each fill buffer
+constexpr uint32_t FLOW_TAIL_BYTES = 512;
+constexpr uint32_t STREAM_BUFFERS = 2 * SCHED_CHUNK_WORDS * 4;  // two fill buffers of a chunk
+constexpr uint32_t FLOW_MAX_C = 8;     // CTAs in a cluster
+constexpr uint32_t FLOW_AHEAD = 8;     // most levels between a send and its deadline
+constexpr uint32_t FLOW_BARS = 32;     // arrival barriers, by level % FLOW_BARS
+constexpr uint32_t FLOW_SKEW = 16;     // levels between the CTAs' progress checks: a sender is at
+                                       // most this far ahead of a receiver, so a deadline is less
+                                       // than FLOW_BARS levels past the receiver's level
+static_assert(FLOW_SKEW + FLOW_AHEAD < FLOW_BARS, "arrival barriers must not wrap");
 
 // 1 / c when c is a positive normal power of two (then x / c == x * (1/c)
 // exactly for every x: both round the same real number), else 0.

@@ -13,6 +13,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <array>
 #include <cstring>
 #include <map>
 #include <tuple>
@@ -87,6 +88,8 @@ Engine::Engine(cudaStream_t stream) : stream_(stream) {
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
     for (auto fn : {k_exec_large<true, true>, k_exec_large<false, true>,
                     k_exec_large<true, false>, k_exec_large<false, false>})
+      cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
+    for (auto fn : {k_exec_flow<true>, k_exec_flow<false>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, v);
     for (auto fn : {k_exec_large<true, true>, k_exec_large<false, true>})
       cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
@@ -588,6 +591,14 @@ int Engine::rebuild_lists() {
     while (b < 31 && (1u << b) < x) ++b;
     return b;
   };
+  std::vector<std::array<uint32_t, 4>> flow_shapes;
+  auto flow_shape = [&](const GroupBody& g) {
+    const std::array<uint32_t, 4> v{g.large_c, g.flow_pos, g.flow_prev, g.flow_rest};
+    const auto it = std::find(flow_shapes.begin(), flow_shapes.end(), v);
+    if (it != flow_shapes.end()) return (uint32_t)(it - flow_shapes.begin());
+    flow_shapes.push_back(v);
+    return (uint32_t)flow_shapes.size() - 1;
+  };
   // A resident schedule takes most of an SM's shared memory (a 32x32 cloth:
   // ~170 KB, one body per SM) where a streamed one leaves room for about
   // three.  Resident schedules win when a launch has no more bodies than SMs
@@ -616,8 +627,10 @@ int Engine::rebuild_lists() {
       const bool use_res =
           gb.res && res_count[std::make_tuple(gb.T, full, log2c(gb.region + gb.res))] <=
                         (size_t)std::max(g_num_sms, 1);
-      // large-body classes are keyed by their cluster layout instead of a bin
-      const uint32_t bin = gb.large_c ? (0x10000u | (gb.large_c << 8) | gb.log2per)
+      // large-body classes are keyed by their cluster layout instead of a bin,
+      // flow classes by their exact shared-memory layout
+      const uint32_t bin = gb.flow_pos ? 0x20000u + flow_shape(gb)
+                           : gb.large_c ? (0x10000u | (gb.large_c << 8) | gb.log2per)
                            : gb.smem ? log2c(gb.region + (use_res ? gb.res : 0u)) : 0u;
       auto key = std::make_tuple(gb.T, gb.smem, full, use_res, bin);
       auto it = cls.find(key);
@@ -639,6 +652,9 @@ int Engine::rebuild_lists() {
       LaunchClass& c = classes_[it->second];
       if (gb.smem) c.region = std::max(c.region, gb.region);
       if (use_res) c.res = std::max(c.res, gb.res);
+      c.flow_pos = gb.flow_pos;
+      c.flow_prev = gb.flow_prev;
+      c.flow_rest = gb.flow_rest;
       c.words = std::max(c.words, reg_.scheds[im.bodies[gb.body].sched].words);
       c.items.push_back(make_uint2(si, gb.body));
     }
@@ -717,6 +733,11 @@ int Engine::rebuild_lists() {
   // size each class to its largest member; a resident class whose largest
   // body and largest schedule do not fit together streams instead
   for (LaunchClass& c : classes_) {
+    if (c.flow_pos) {  // the largest fills (to 64 KB) beside the body
+      const uint32_t used = c.flow_pos + c.flow_prev + c.flow_rest + FLOW_TAIL_BYTES;
+      const uint32_t room = (uint32_t)std::max((int)g_smem_optin - (int)used, 0) / 2 & ~15u;
+      c.fill = std::min(room, 65536u);
+    }
     if (c.large_c) continue;  // one body per cluster, shared memory set by its layout
     if (c.res && (size_t)c.region + c.res + GROUP_TAIL_BYTES > (size_t)g_smem_optin) c.res = 0;
     // streamed: one 16 KB chunk per fill, or for launches with no more bodies
@@ -889,11 +910,18 @@ int Engine::launch_all(bool profiling) {
   // one launch of a group class over n work items starting at L
   auto launch_class = [&](const LaunchClass& c, const uint2* L, uint32_t n, uint32_t cur,
                           uint32_t sub, cudaStream_t st) {
-    if (c.large_c) {  // large-body executor: one cluster of large_c CTAs per body
+    if (c.large_c) {  // flow or large-body executor: one cluster of large_c CTAs per body
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = dim3(n * c.large_c);
       cfg.blockDim = dim3(c.T);
-      cfg.dynamicSmemBytes = (size_t)(c.full ? 16u : 8u) << c.log2per;
+      FlowLayout Y;
+      Y.prev = c.flow_pos;
+      Y.rest = Y.prev + c.flow_prev;
+      Y.fill = Y.rest + c.flow_rest;  // (multiples of 16)
+      Y.fill_bytes = c.fill;
+      Y.tail = Y.fill + 2u * c.fill;
+      cfg.dynamicSmemBytes = c.flow_pos ? Y.tail + FLOW_TAIL_BYTES
+                                        : (size_t)(c.full ? 16u : 8u) << c.log2per;
       cfg.stream = st;
       cudaLaunchAttribute at[1];
       at[0].id = cudaLaunchAttributeClusterDimension;
@@ -902,6 +930,11 @@ int Engine::launch_all(bool profiling) {
       at[0].val.clusterDim.z = 1;
       cfg.attrs = at;
       cfg.numAttrs = c.large_c > 1 ? 1u : 0u;
+      if (c.flow_pos) {
+        lk(cudaLaunchKernelEx(&cfg, c.full ? k_exec_flow<true> : k_exec_flow<false>, W, SC, L, n,
+                              c.large_c, Y, cur, sub));
+        return;
+      }
       void (*kl)(const DWorld*, DScheds, const uint2*, uint32_t, uint32_t, uint32_t, uint32_t,
                  uint32_t) =
           c.full ? (c.large_c > 1 ? k_exec_large<true, true> : k_exec_large<true, false>)
@@ -931,7 +964,8 @@ int Engine::launch_all(bool profiling) {
   auto groups = [&](bool full, uint32_t cur, uint32_t sub) {
     for (const LaunchClass& c : classes_) {
       if (c.full != full || c.items.empty()) continue;
-      const char* name = c.large_c ? (full ? "exec_large_full" : "exec_large_links")
+      const char* name = c.flow_pos ? (full ? "exec_flow_full" : "exec_flow_links")
+                         : c.large_c ? (full ? "exec_large_full" : "exec_large_links")
                          : full ? (c.smem ? "exec_groups_full_smem" : "exec_groups_full_global")
                                 : (c.smem ? "exec_groups_links_smem" : "exec_groups_links_global");
       const cudaStream_t st = branch();

@@ -68,6 +68,11 @@ struct SchedRegistry {
   // a whole level (or what of it fits a chunk)
   uint32_t get(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I, bool full,
                bool group, const PlanTuning& t);
+  // the flow schedule of a large body over C CTAs (np <= 65535); NONE when it
+  // does not fit the op format
+  static constexpr uint32_t NONE = 0xFFFFFFFFu;
+  uint32_t get_flow(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I, bool full,
+                    uint32_t C);
 };
 
 struct GroupBody {
@@ -78,6 +83,9 @@ struct GroupBody {
   bool smem;
   uint32_t large_c = 0;  // large-body executor: CTAs in the body's cluster (0: not used)
   uint32_t log2per = 0;  // large-body executor: log2 of the particles per CTA
+  // flow executor (large_c CTAs): bytes of positions, previous positions and
+  // link parameters in each CTA's shared memory (pos 0: not a flow body)
+  uint32_t flow_pos = 0, flow_prev = 0, flow_rest = 0;
 };
 
 
@@ -136,6 +144,7 @@ struct LaunchClass {
   bool smem, full;
   bool skip = false;  // more bodies than SMs: idle warps skip a round's work
   uint32_t large_c = 0, log2per = 0;  // large-body executor class (large_c CTAs per body)
+  uint32_t flow_pos = 0, flow_prev = 0, flow_rest = 0;  // flow executor class: its bodies'
   std::vector<uint2> items;
   size_t dev_off = 0;  // offset (in uint2) into the device list buffer
 };

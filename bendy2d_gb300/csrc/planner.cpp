@@ -210,6 +210,186 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
   return id;
 }
 
+uint32_t SchedRegistry::get_flow(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I,
+                                 bool full, uint32_t C) {
+  std::string key;
+  const uint32_t hdr[8] = {np, nl, S, I, (full ? 1u : 0u) | 4u, C, 0u, 0u};
+  key.resize(sizeof(hdr) + (size_t)nl * 8);
+  std::memcpy(&key[0], hdr, sizeof(hdr));
+  if (nl) std::memcpy(&key[sizeof(hdr)], links, (size_t)nl * 8);
+  auto it = index.find(key);
+  if (it != index.end()) return it->second;
+  if (np > 65535u || C < 2 || C > FLOW_MAX_C || np < C) return NONE;
+
+  // CTA r integrates particles [np*r/C, np*(r+1)/C) and solves the links
+  // whose first endpoint is one of them
+  std::vector<uint32_t> own(C + 1);
+  for (uint32_t r = 0; r <= C; ++r) own[r] = (uint32_t)((uint64_t)np * r / C);
+  std::vector<uint8_t> cta(np);
+  for (uint32_t r = 0; r < C; ++r)
+    for (uint32_t p = own[r]; p < own[r + 1]; ++p) cta[p] = (uint8_t)r;
+  std::vector<uint32_t> lidx(nl);  // link -> its index among its CTA's links
+  std::vector<std::vector<uint32_t>> mine(C);
+  for (uint32_t k = 0; k < nl; ++k) {
+    std::vector<uint32_t>& m = mine[cta[links[k].x]];
+    lidx[k] = (uint32_t)m.size();
+    if (m.size() > 65535u) return NONE;
+    m.push_back(k);
+  }
+  // ops in sequence, with their levels; of each op, where its particles go next
+  struct Op { uint32_t id, level; uint8_t cta, to[2]; };
+  const uint32_t nsub = full ? S : 1u;
+  std::vector<Op> seq;
+  seq.reserve((size_t)nsub * ((size_t)I * nl + (full ? np : 0)));
+  struct Use { uint32_t op; uint8_t end; };  // a particle's latest use
+  std::vector<Use> last(np, Use{NONE, 0});
+  std::vector<uint32_t> depth(np, 0), first(np, NONE), lo(C, NONE), hi(C, 0);
+  std::vector<std::vector<uint32_t>> expect(C);
+  uint32_t nlvl = 0;
+  auto use = [&](uint32_t p, uint32_t op, uint8_t end) {
+    Op& o = seq[op];
+    lo[o.cta] = std::min(lo[o.cta], p);
+    hi[o.cta] = std::max(hi[o.cta], p + 1);
+    const Use u = last[p];
+    if (u.op == NONE) {
+      first[p] = o.cta;
+    } else if (seq[u.op].cta != o.cta) {
+      const uint32_t d = std::min(o.level - seq[u.op].level, FLOW_AHEAD);
+      seq[u.op].to[u.end] = (uint8_t)(1u | (o.cta << 1) | ((d - 1u) << 4));
+      std::vector<uint32_t>& e = expect[o.cta];
+      const uint32_t at = seq[u.op].level + d;
+      if (e.size() <= at) e.resize(at + 64, 0);
+      ++e[at];
+    }
+    last[p] = Use{op, end};
+    depth[p] = o.level + 1;
+    nlvl = std::max(nlvl, o.level + 1);
+  };
+  for (uint32_t s = 0; s < nsub; ++s) {
+    for (uint32_t it2 = 0; it2 < I; ++it2)
+      for (uint32_t k = 0; k < nl; ++k) {
+        const uint32_t a = links[k].x, b = links[k].y, op = (uint32_t)seq.size();
+        seq.push_back(Op{k, std::max(depth[a], depth[b]), cta[a], {0, 0}});
+        use(a, op, 0);
+        use(b, op, 1);
+      }
+    if (full)
+      for (uint32_t p = 0; p < np; ++p) {
+        seq.push_back(Op{OP_INTEG | p, depth[p], cta[p], {0, 0}});
+        use(p, (uint32_t)seq.size() - 1, 0);
+      }
+  }
+  // by CTA, level, and kind: links that send, other links, integrate ops
+  auto kind = [](const Op& o) { return o.id & OP_INTEG ? 2u : (o.to[0] | o.to[1]) & 1u ? 0u : 1u; };
+  std::vector<uint32_t> count((size_t)C * nlvl * 3 + 1, 0);
+  auto bin = [&](const Op& o) { return ((size_t)o.cta * nlvl + o.level) * 3 + kind(o); };
+  for (const Op& o : seq) ++count[bin(o) + 1];
+  for (size_t i = 1; i < count.size(); ++i) count[i] += count[i - 1];
+  std::vector<uint32_t> order(seq.size());
+  {
+    std::vector<uint32_t> at(count.begin(), count.end() - 1);
+    for (uint32_t i = 0; i < seq.size(); ++i) order[at[bin(seq[i])]++] = i;
+  }
+  uint32_t max_link = 0, max_integ = 0;
+  for (size_t g = 0; g < (size_t)C * nlvl; ++g) {
+    max_link = std::max(max_link, count[3 * g + 2] - count[3 * g]);
+    max_integ = std::max(max_integ, count[3 * g + 3] - count[3 * g + 2]);
+  }
+  DSched d{};
+  d.nlvl = nlvl;
+  d.nops = (uint32_t)seq.size();
+  d.tl = std::min(std::max((max_link + 31u) & ~31u, 32u), 512u);
+  d.ti = max_integ ? std::min((max_integ + 31u) & ~31u, 256u) : 0u;
+  d.chunk0 = (uint32_t)chunk_off.size();
+  std::vector<uint32_t> rec((size_t)C * FLOW_REC_WORDS, 0);
+  for (uint32_t r = 0; r < C; ++r) {
+    uint32_t* R = &rec[(size_t)r * FLOW_REC_WORDS];
+    if (lo[r] == NONE) lo[r] = own[r], hi[r] = own[r] + 1;
+    R[FR_CHUNK0] = (uint32_t)chunk_off.size();
+    R[FR_LO] = lo[r];
+    R[FR_WINDOW] = hi[r] - lo[r];
+    R[FR_OWN0] = own[r];
+    R[FR_OWN1] = own[r + 1];
+    std::vector<uint32_t> words, ops;  // of the open chunk: rounds; op indices in seq
+    auto flush = [&](uint32_t next_level) {
+      while (stream.size() % 4) stream.push_back(0);
+      chunk_off.push_back((uint32_t)stream.size());
+      const size_t at = stream.size();
+      stream.push_back((uint32_t)words.size());
+      stream.insert(stream.end(), words.begin(), words.end());
+      const uint32_t end = (uint32_t)ops.size();
+      stream.insert(stream.end(), 2, end | (end << 11) | ((next_level % 32u) << 22));
+      if ((stream.size() - at) % 2) stream.push_back(0);
+      for (uint32_t i : ops) {
+        const Op& o = seq[i];
+        if (o.id & OP_INTEG) {
+          stream.push_back((o.id & ~OP_INTEG) * 0x10001u);
+          stream.push_back((uint32_t)o.to[0] << 16);
+        } else {
+          stream.push_back(links[o.id].x | (links[o.id].y << 16));
+          stream.push_back(lidx[o.id] | ((uint32_t)o.to[0] << 16) | ((uint32_t)o.to[1] << 23));
+        }
+      }
+      stream.push_back(lo[r] * 0x10001u);
+      stream.push_back(0);
+      while ((stream.size() - at) % 4) stream.push_back(0);
+      chunk_len.push_back((uint32_t)(stream.size() - at));
+      if (chunk_len.back() > SCHED_CHUNK_WORDS) std::abort();
+      words.clear();
+      ops.clear();
+    };
+    auto room = [&]() -> uint32_t {  // ops that fit beside one more round and the last op
+      const size_t used = sched_head_words((uint32_t)words.size() + 1) + 2 * ops.size() + 2 + 3;
+      return used + 2 > SCHED_CHUNK_WORDS ? 0u : (uint32_t)(SCHED_CHUNK_WORDS - used) / 2;
+    };
+    for (uint32_t l = 0; l < nlvl; ++l) {
+      const size_t g = (size_t)r * nlvl + l;
+      uint32_t lk = count[3 * g], in = count[3 * g + 2];
+      const uint32_t le = in, ie = count[3 * g + 3];
+      do {  // a level without ops here is an empty round
+        const uint32_t want_l = std::min(le - lk, d.tl), want = want_l + (ie - in);
+        if (room() < std::max(want, 1u) && !words.empty()) flush(l);
+        const uint32_t tl = std::min(want_l, room()), ti = std::min(ie - in, room() - tl);
+        ops.insert(ops.end(), order.begin() + lk, order.begin() + lk + tl);
+        const uint32_t lend = (uint32_t)ops.size();
+        ops.insert(ops.end(), order.begin() + in, order.begin() + in + ti);
+        words.push_back(lend | ((uint32_t)ops.size() << 11) | ((l % 32u) << 22));
+        lk += tl;
+        in += ti;
+      } while (lk < le || in < ie);
+    }
+    flush(nlvl);
+    R[FR_NCHUNKS] = (uint32_t)chunk_off.size() - R[FR_CHUNK0];
+  }
+  d.nchunks = (uint32_t)chunk_off.size() - d.chunk0;
+  auto list = [&](const std::vector<uint32_t>& v, uint32_t* at, uint32_t* n) {
+    *at = (uint32_t)stream.size();
+    *n = (uint32_t)v.size();
+    stream.insert(stream.end(), v.begin(), v.end());
+  };
+  for (uint32_t r = 0; r < C; ++r) {
+    uint32_t* R = &rec[(size_t)r * FLOW_REC_WORDS];
+    list(mine[r], &R[FR_LINKS], &R[FR_NLINKS]);
+    std::vector<uint32_t> load, store;
+    for (uint32_t p = 0; p < np; ++p) {
+      if (first[p] == r) load.push_back(p);
+      if (first[p] != NONE && seq[last[p].op].cta == r) store.push_back(p);
+    }
+    list(load, &R[FR_LOAD], &R[FR_NLOAD]);
+    list(store, &R[FR_STORE], &R[FR_NSTORE]);
+    expect[r].resize(nlvl, 0);
+    list(expect[r], &R[FR_EXPECT], &R[FR_NLEVELS]);
+  }
+  while (stream.size() % 4) stream.push_back(0);
+  d.off = (uint32_t)stream.size();
+  d.words = (uint32_t)rec.size();
+  stream.insert(stream.end(), rec.begin(), rec.end());
+  const uint32_t id = (uint32_t)scheds.size();
+  scheds.push_back(d);
+  index.emplace(std::move(key), id);
+  return id;
+}
+
 // Bounds check of a finished image: every index a kernel dereferences must
 // land inside the world's arrays.  Runs on every plan (linear in the size of
 // the world); a failure is a planner bug and stops the world from reaching
@@ -250,8 +430,27 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
         (size_t)S.off + S.words > reg.stream.size())
       return bad("schedule range");
     if (g.smem && (!B.local || B.np > 65535u)) return bad("shared-memory body needs local links");
-    if (g.large_c && (g.smem || !B.local || g.large_c > 16u || g.log2per > 14u ||
-                      (size_t)g.large_c << g.log2per < B.np || g.T > 1024u))
+    if (g.flow_pos) {  // the flow executor's records
+      if (g.smem || !B.local || g.large_c < 2 || g.large_c > FLOW_MAX_C || B.np > 65535u ||
+          S.words != g.large_c * FLOW_REC_WORDS || g.T != S.tl + S.ti + 32u || S.tl > 512u ||
+          S.ti > 256u)
+        return bad("flow executor layout");
+      for (uint32_t r = 0; r < g.large_c; ++r) {
+        const uint32_t* R = &reg.stream[S.off + r * FLOW_REC_WORDS];
+        if ((size_t)R[FR_CHUNK0] + R[FR_NCHUNKS] > reg.chunk_off.size() ||
+            R[FR_LO] + R[FR_WINDOW] > B.np || 8u * R[FR_WINDOW] > g.flow_pos || R[FR_OWN1] > B.np ||
+            R[FR_NLEVELS] != S.nlvl)
+          return bad("flow executor record");
+        for (uint32_t f : {FR_LINKS, FR_LOAD, FR_STORE, FR_EXPECT})
+          if ((size_t)R[f] + R[f + 1] > reg.stream.size()) return bad("flow executor list");
+        for (uint32_t i = 0; i < R[FR_NLINKS]; ++i)
+          if (reg.stream[R[FR_LINKS] + i] >= B.nl) return bad("flow executor link");
+        for (uint32_t f : {FR_LOAD, FR_STORE})
+          for (uint32_t i = 0; i < R[f + 1]; ++i)
+            if (reg.stream[R[f] + i] - R[FR_LO] >= R[FR_WINDOW]) return bad("flow executor particle");
+      }
+    } else if (g.large_c && (g.smem || !B.local || g.large_c > 16u || g.log2per > 14u ||
+                             (size_t)g.large_c << g.log2per < B.np || g.T > 1024u))
       return bad("large-body executor layout");
     if (g.res && (!g.smem || g.res != S.words * 4u)) return bad("resident schedule size");
     if (g.T < 32 || g.T % 32) return bad("group size");
@@ -487,12 +686,43 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     const size_t state = (full ? 16u : 8u) * (size_t)B.np;
     const bool smem = align16(state + 8u * (size_t)B.nl) <= tune.smem_max && B.np <= 65535u;
     const size_t region = align16(state + (B.flags & BODY_UNIT ? 4u : 8u) * (size_t)B.nl);
-    B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, smem, tune);
+    // A body over one CTA's shared memory: the flow executor, over as many CTAs
+    // as give each ~200 ops a level, at least as many as hold it; failing that
+    // (more than 65,535 particles, or too much for large_max CTAs) the
+    // large-body executor below, and beyond it the group executor from
+    // global memory.
+    uint32_t flow_c = 0, flow[3] = {0, 0, 0};
+    if (!smem && tune.large_max >= 2 && B.np <= 65535u) {
+      const double depth_est = (double)at.size() - 1.0;  // levels of one pass
+      const double wide = (double)B.nl / std::max(depth_est, 1.0) * (full ? (double)P.S * P.I : P.I);
+      uint32_t c = (uint32_t)std::min(std::max(wide / 400.0, 2.0), (double)FLOW_MAX_C);
+      const uint32_t most = std::min(tune.large_max, FLOW_MAX_C);
+      for (c = std::min(c, most); c <= most && !flow_c; ++c) {
+        // (what it takes at the least, before its schedule is built)
+        const size_t least = (state + (B.flags & BODY_UNIT ? 4u : 8u) * (size_t)B.nl) / c;
+        if (least + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
+        const uint32_t id = reg.get_flow(loc.data(), B.nl, B.np, P.S, P.I, full, c);
+        if (id == SchedRegistry::NONE) break;
+        uint32_t need[3] = {0, 0, 0};
+        for (uint32_t r = 0; r < c; ++r) {
+          const uint32_t* R = &reg.stream[reg.scheds[id].off + r * FLOW_REC_WORDS];
+          need[0] = std::max(need[0], 8u * R[FR_WINDOW]);
+          if (full) need[1] = std::max(need[1], 8u * (R[FR_OWN1] - R[FR_OWN0]));
+          need[2] = std::max(need[2], (B.flags & BODY_UNIT ? 4u : 8u) * R[FR_NLINKS]);
+        }
+        for (uint32_t& v : need) v = (uint32_t)align16(v);
+        if ((size_t)need[0] + need[1] + need[2] + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
+        flow_c = c;
+        std::copy(need, need + 3, flow);
+        B.sched = id;
+      }
+    }
+    if (!flow_c) B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, smem, tune);
     const DSched& S = reg.scheds[B.sched];
     const float avg = S.nlvl ? (float)S.nops / (float)S.nlvl : 1.0f;
     uint32_t T = pow2ceil((uint32_t)(avg / tune.width_per_thread + 0.999f));
     T = std::min(std::max(T, tune.t_min), tune.t_max);
-    if (smem) T = S.tl + S.ti;
+    if (smem || flow_c) T = S.tl + S.ti;
     // the whole schedule resident in shared memory when it fits beside the body
     uint32_t res = 0;
     if (smem && tune.resident) {
@@ -507,7 +737,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // through the caches; beyond that the group executor runs it from
     // global memory.
     uint32_t large_c = 0, log2per = 0, TL = T;
-    if (!smem && tune.large_max > 0 && B.np > 0) {
+    if (!smem && !flow_c && tune.large_max > 0 && B.np > 0) {
       const uint32_t cap_log2 = full ? 13u : 14u;
       uint32_t l2 = 0;
       while (l2 < cap_log2 && (1u << l2) < B.np) ++l2;
@@ -518,6 +748,10 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
         const float w = avg / (tune.width_per_thread * (float)c);
         TL = std::min<uint32_t>(1024u, std::max<uint32_t>(64u, pow2ceil((uint32_t)(w + 0.999f))));
       }
+    }
+    if (flow_c) {
+      large_c = flow_c;
+      TL = T + 32;  // and the control warp
     }
     const bool local = smem || large_c > 0;
     B.local = local ? 1u : 0u;
@@ -530,6 +764,9 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     GroupBody gbody{id, large_c ? TL : T, smem ? (uint32_t)region : 0u, res, smem};
     gbody.large_c = large_c;
     gbody.log2per = log2per;
+    gbody.flow_pos = flow[0];
+    gbody.flow_prev = flow[1];
+    gbody.flow_rest = flow[2];
     im.groups.push_back(gbody);
     im.stats.group_bodies++;
     if (large_c) im.stats.large_bodies++;
