@@ -32,7 +32,7 @@ SPACE = {
     "resident": [0, 1],
     "stage_frac": [0.4, 0.67, 1.01],
     "bucket_factor": [1.0, 2.0, 4.0],
-    "collide_thread_min": [0, 131072, 1 << 30],
+    "collide_thread_min": [0, 81920, 1 << 30],
     "grid_slot_max": [0, 262144, 1 << 30],
 }
 # The planner's defaults for the tunables above (PlanTuning in
@@ -46,7 +46,7 @@ DEFAULTS = {
     "resident": 1,
     "stage_frac": 1.01,
     "bucket_factor": 2.0,
-    "collide_thread_min": 131072,
+    "collide_thread_min": 81920,
     "grid_slot_max": 262144,
 }
 # tunables that matter for batches of chain-like worlds (rings), where the

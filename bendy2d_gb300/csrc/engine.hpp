@@ -46,7 +46,7 @@ struct PlanTuning {
                                     // with positions forwarded in registers ordinary packs
                                     // run the longest chains faster)
   float bucket_factor = 2.0f;       // collision-grid buckets per world: pow2 >= this x particles
-  uint32_t collide_thread_min = 131072;  // particles in the collide pass from which it runs
+  uint32_t collide_thread_min = 81920;  // particles in the collide pass from which it runs
                                          // one thread per particle (else three lanes each)
   uint32_t large_max = 8;           // largest cluster of the large-body executor (0: bodies
                                     // over one CTA's shared memory run from global memory)
