@@ -730,6 +730,48 @@ int Engine::rebuild_lists() {
     B2D_CUDA(cudaMemcpyAsync(d_worlds_ + rec_lo, &h_worlds_[rec_lo],
                              (size_t)(rec_hi - rec_lo + 1) * sizeof(DWorld),
                              cudaMemcpyHostToDevice, stream_));
+  // One launch for all the group classes of a pass (resident and streamed
+  // apart) whose bodies can each have an SM to themselves: a launch's position
+  // in the graph costs more than the threads that smaller bodies leave idle
+  // (40 request worlds, 11 classes in each link pass: an update of eight
+  // sub-steps 354 us, as one launch a pass 294 us).  Where other executors run
+  // beside them, half the SMs stay theirs.
+  if (!plain_) {
+    for (const bool full : {false, true})
+      for (const bool res : {false, true}) {
+        const size_t rigid = (full ? rigid_full_ : rigid_ext_).size(), sms = std::max(g_num_sms, 1);
+        bool others = !(full ? sfull_all : slinks_all).empty();
+        std::vector<size_t> cand;
+        for (size_t c = 0; c < classes_.size(); ++c) {
+          if (classes_[c].full != full) continue;
+          if (!classes_[c].smem || classes_[c].large_c) others = true;
+          else if ((classes_[c].res != 0) == res) cand.push_back(c);
+        }
+        std::stable_sort(cand.begin(), cand.end(),
+                         [&](size_t a, size_t b) { return classes_[a].T > classes_[b].T; });
+        const size_t room = (sms - std::min(sms, rigid)) / (others ? 2 : 1);
+        LaunchClass* into = nullptr;
+        for (const size_t k : cand) {
+          LaunchClass& c = classes_[k];
+          if (c.items.size() + (into ? into->items.size() : 0) > room) continue;
+          if (into && (size_t)std::max(into->region, c.region) + std::max(into->res, c.res) +
+                          GROUP_TAIL_BYTES > (size_t)g_smem_optin)
+            continue;
+          if (!into) {
+            into = &c;
+            continue;
+          }
+          into->region = std::max(into->region, c.region);
+          into->res = std::max(into->res, c.res);
+          into->words = std::max(into->words, c.words);
+          into->items.insert(into->items.end(), c.items.begin(), c.items.end());
+          c.items.clear();
+        }
+      }
+    classes_.erase(std::remove_if(classes_.begin(), classes_.end(),
+                                  [](const LaunchClass& c) { return c.items.empty(); }),
+                   classes_.end());
+  }
   // size each class to its largest member; a resident class whose largest
   // body and largest schedule do not fit together streams instead
   for (LaunchClass& c : classes_) {
