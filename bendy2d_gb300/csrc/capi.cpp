@@ -578,12 +578,8 @@ int b2d_state_upload_async(b2d_solver* s, const void* src) {
   CHECK_S(s);
   int st = ensure_placed(s);
   if (st != OK) return st;
-  void* d;
-  size_t n;
-  st = s->eng->state_span(s->slot, &d, &n);
-  if (st != OK) return st;
-  if (cudaMemcpyAsync(d, src, n, cudaMemcpyHostToDevice, s->eng->stream()) != cudaSuccess)
-    return fail(ERR_CUDA, "state upload failed");
+  st = s->eng->copy_state(s->slot, const_cast<void*>(src), true);
+  if (st != OK) return st == ERR_CUDA ? fail(ERR_CUDA, "state upload failed") : st;
   s->host_stale = true;
   return OK;
 }
@@ -591,13 +587,8 @@ int b2d_state_download_async(b2d_solver* s, void* dst) {
   CHECK_S(s);
   int st = ensure_placed(s);
   if (st != OK) return st;
-  void* d;
-  size_t n;
-  st = s->eng->state_span(s->slot, &d, &n);
-  if (st != OK) return st;
-  if (cudaMemcpyAsync(dst, d, n, cudaMemcpyDeviceToHost, s->eng->stream()) != cudaSuccess)
-    return fail(ERR_CUDA, "state download failed");
-  return OK;
+  st = s->eng->copy_state(s->slot, dst, false);
+  return st == ERR_CUDA ? fail(ERR_CUDA, "state download failed") : st;
 }
 
 int b2d_get_plan_stats(b2d_solver* s, b2d_plan_stats* out) {

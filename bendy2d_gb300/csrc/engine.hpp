@@ -178,6 +178,8 @@ class Engine {
   // raw state prefix (pos, prev, circles, polygons) of a world, for end-to-end
   // transfers from and to pinned host memory
   int state_span(uint32_t slot, void** dptr, size_t* bytes);
+  // the world's state from or to host memory, in the engine's stream's order
+  int copy_state(uint32_t slot, void* host, bool up);
   int sync();
   void set_stream(cudaStream_t s);
   cudaStream_t stream() const { return stream_; }
