@@ -578,6 +578,7 @@ int Engine::rebuild_lists() {
   smax_ext_ = 0;
   any_odd_ext_ = false;
   any_pp_ = false;
+  any_rigid_contacts_ = false;
   any_count_ = false;
   size_t np_ext = 0;
   size_t nbuckets = 0, np_pp = 0;
@@ -704,6 +705,7 @@ int Engine::rebuild_lists() {
       }
       smax_ext_ = std::max(smax_ext_, im.params.S);
       any_odd_ext_ |= (im.params.S & 1u) != 0u;
+      any_rigid_contacts_ |= (im.params.flags & (COLLIDE_PC | COLLIDE_PPOLY)) != 0u;
       if (im.params.flags & COLLIDE_PP) {
         any_pp_ = true;
         // this world's bucket range: a power of two >= 2 x its particles
@@ -1165,21 +1167,25 @@ int Engine::launch_all(bool profiling) {
     }
     if (nre) edge(ax, stream_);
     if (nch) timed("collide_integrate", [&] {
-      if (grid_slotted_ || !any_pp_) {
+      auto collide = [&](const auto& grid, auto rigid) {
+        using GRID = std::decay_t<decltype(grid)>;
+        constexpr bool RIGID = decltype(rigid)::value;
+        const uint32_t nct = nch * COLLIDE_CTAS;
         if (collide_per_particle_)
-          lk(launch_k(k_collide_particle<DSlots>, dim3(nch), dim3(COLLIDE_P_THREADS), 0, stream_,
-                      !profiling, W, GS, CH, nch, cur, s));
-        else
-          lk(launch_k(k_collide_integrate<DSlots>, dim3(nch * COLLIDE_CTAS),
-                      dim3(COLLIDE_THREADS), 0, stream_, !profiling, W, GS, CH, nch, cur, s));
-      } else {
-        if (collide_per_particle_)
-          lk(launch_k(k_collide_particle<DGrid>, dim3(nch), dim3(COLLIDE_P_THREADS), 0, stream_,
-                      !profiling, W, GR, CH, nch, cur, s));
-        else
-          lk(launch_k(k_collide_integrate<DGrid>, dim3(nch * COLLIDE_CTAS),
-                      dim3(COLLIDE_THREADS), 0, stream_, !profiling, W, GR, CH, nch, cur, s));
-      }
+          lk(launch_k(k_collide_particle<GRID, RIGID>, dim3(nch), dim3(COLLIDE_P_THREADS), 0, stream_,
+                      !profiling, W, grid, CH, nch, cur, s));
+        else  // six CTAs an SM where five would leave a few for a second wave
+          lk(launch_k(nct <= 5u * (uint32_t)std::max(g_num_sms, 1) ? k_collide_integrate<GRID, 5, RIGID>
+                                                                 : k_collide_integrate<GRID, 6, RIGID>,
+                      dim3(nct), dim3(COLLIDE_THREADS), 0, stream_, !profiling, W, grid, CH, nch,
+                      cur, s));
+      };
+      auto over = [&](const auto& grid) {
+        if (any_rigid_contacts_) collide(grid, std::true_type{});
+        else collide(grid, std::false_type{});
+      };
+      if (grid_slotted_ || !any_pp_) over(GS);
+      else over(GR);
     });
     if (nre) edge(stream_, ax);
   }

@@ -276,6 +276,7 @@ class Engine {
   void build_packs(std::vector<uint2>& in, bool full, SerialPacks* out, std::vector<uint2>& rest,
                    bool allow_large);
   std::vector<WorldLaunch> wlaunch_;
+  bool any_rigid_contacts_ = false;  // a world whose particles meet circles or polygons
   bool any_pp_ = false;
   bool any_count_ = false;  // a world with particle collisions needs the insert (count) kernel
   bool collide_per_particle_ = false;  // k_collide_particle instead of k_collide_integrate

@@ -194,7 +194,7 @@ extern "C" int b2d_collide_substeps_noalloc(float* d_pos_xy, float* d_prev_xy, s
     if ((e = launch(k_grid_scatter, nch, CHUNK, st, (const DWorld*)dW, G, (const uint2*)chunks,
                     nch, cur, s)) != cudaSuccess)
       return bad(e, "scatter launch");
-    if ((e = launch(k_collide_integrate<DGrid>, nch * COLLIDE_CTAS, COLLIDE_THREADS, st,
+    if ((e = launch(k_collide_integrate<DGrid, 5, true>, nch * COLLIDE_CTAS, COLLIDE_THREADS, st,
                     (const DWorld*)dW, G, (const uint2*)chunks, nch, cur, s)) != cudaSuccess)
       return bad(e, "collide launch");
   }
