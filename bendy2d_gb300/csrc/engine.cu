@@ -992,11 +992,13 @@ int Engine::launch_all(bool profiling) {
     const size_t sm = (size_t)c.G * (c.region + sb + GROUP_TAIL_BYTES);
     const uint32_t rg = c.smem ? c.region : 0u;
     // The sub-step pipeline's main-stream link launch follows the previous
-    // sub-step's collide kernel programmatically when its schedules are
-    // resident: at most one CTA per SM waits early, leaving the SMs the
-    // circle/polygon branch needs.  (Large streamed launches started early
-    // filled every SM and delayed that branch: 18 % slower on 1,024 bodies.)
-    const bool pdl = !profiling && !c.full && c.res && st == stream_;
+    // sub-step's collide kernel programmatically while the early CTAs leave
+    // SMs half free for the circle/polygon branch, which starts after them:
+    // up to one and a half bodies an SM.  (Cloths of 32x32, streamed, an update
+    // of 20 sub-steps: 100 bodies 1015 -> 941 us, 200 1282 -> 1220, but 260
+    // 1544 -> 1671; 1,024 bodies were 18 % slower.)
+    const bool pdl = !profiling && !c.full && st == stream_ &&
+                     2 * (size_t)n <= 3 * (size_t)std::max(g_num_sms, 1);
     void (*k)(const DWorld*, DScheds, const uint2*, uint32_t, uint32_t, uint32_t, uint32_t,
               uint32_t, uint32_t, uint32_t, uint32_t*, uint2*, DSlots) =
         c.res ? (c.full ? k_exec_groups<true, true, true, false> : k_exec_groups<false, true, true, false>)
