@@ -49,12 +49,25 @@ struct DBody {
 // Every rest length is below 2^100 in magnitude: the fused-arithmetic link
 // solve (kernels.cuh, link_solve_fused) may run.
 // A serial executor's body.
-enum : uint32_t { BODY_UNIT = 1u, BODY_RANGE = 2u, BODY_SERIAL = 4u };
+// One whose consecutive links (within each half) share one particle: it is
+// carried from link to link in registers.
+enum : uint32_t { BODY_UNIT = 1u, BODY_RANGE = 2u, BODY_SERIAL = 4u, BODY_CARRY = 8u };
 constexpr uint32_t BODY_LAG_SHIFT = 8;
 // Mark on a link endpoint of a serial body in two chains: no later link of
 // the pass moves this particle (it is integrated right after).
 constexpr uint32_t LINK_FINAL = 0x80000000u;
+// A carried body's record {x, y, ..}: y is the endpoint that the link before
+// hands on, x the other one.  On x: the link is (y, x), not (x, y).  On y: y is
+// handed on once more, else x is.
+constexpr uint32_t LINK_SWAPPED = 0x40000000u, LINK_KEEP = 0x40000000u;
+constexpr uint32_t LINK_INDEX = 0x3FFFFFFFu;
 constexpr uint32_t NO_FIRST = 0xFFFFFFFFu;
+
+// a serial record's endpoints in the link's order
+__host__ __device__ inline uint2 record_ends(const uint4& r) {
+  const uint32_t x = r.x & LINK_INDEX, y = r.y & LINK_INDEX;
+  return (r.x & LINK_SWAPPED) ? uint2{y, x} : uint2{x, y};
+}
 
 struct DPoly {
   uint32_t v0, nv;       // vertices
@@ -166,7 +179,7 @@ struct DWorld {
   float* lrest;
   float* lstiff;
   uint4* lrec;           // serial bodies' links: {a, b, rest bits, stiffness bits}, endpoints
-                         // body-local with their LINK_FINAL marks
+                         // body-local with their LINK_ marks
   // circles (src/circle.rs:4-8) and circle links
   float2* cpos; float2* cprev; float2* cacc;
   float* crad; uint32_t* cstatic;

@@ -415,9 +415,7 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
       return bad("body first particle");
     const uint32_t lim = B.local ? B.np : P.np;
     for (uint32_t k = 0; k < B.nl; ++k) {
-      const uint2 e = serial ? make_uint2(im.lrec[B.l0 + k].x & ~LINK_FINAL,
-                                          im.lrec[B.l0 + k].y & ~LINK_FINAL)
-                             : im.lab[B.l0 + k];
+      const uint2 e = serial ? record_ends(im.lrec[B.l0 + k]) : im.lab[B.l0 + k];
       if (e.x >= lim || e.y >= lim || e.x == e.y) return bad("link endpoint");
     }
   }
@@ -519,9 +517,9 @@ PassDepth pass_depth(const WorldHost& w, const Comp& c, float enough, std::vecto
 // Whether the second half of a serial body's links can run beside the first
 // half of the next pass, a lag behind it: step j solves link j of the second
 // half and link j - lag of the next first half; a particle is integrated a step
-// after the link that moves it last.  So every particle of first-half link i
-// must have been moved for the last time in the pass by step i + lag - 2, and
-// every particle must be moved by some link of the second half.  A link integrates one particle; only the last, which
+// after the link that moves it last, and read a step before its link.  So every
+// particle of first-half link i must have been moved for the last time in the
+// pass by step i + lag - 3, and every particle must be moved by some link of the second half.  A link integrates one particle; only the last, which
 // moves both of its particles last, has a step more for the other.  Taken when
 // the lag is at most a quarter of the half: then B.sched is the first half's
 // length, the lag is in B.flags, and the last link of the pass that moves a
@@ -537,11 +535,11 @@ void split_chain(DBody& B, uint4* ab) {
     if (l == NONE) return;
   for (uint32_t j = 0; j + 1 < nb; ++j)
     if (last[ab[m + j].x] == j && last[ab[m + j].y] == j) return;
-  const uint32_t other = ab[B.nl - 1].y;  // integrated a step after the last link
+  const uint4 end = ab[B.nl - 1];  // one of its particles is integrated a step after it
   uint32_t lag = 1;
   for (uint32_t i = 0; i < m; ++i) {
-    uint32_t l = std::max(last[ab[i].x], last[ab[i].y]) + 2u;
-    if (ab[i].x == other || ab[i].y == other) l = nb + 2u;
+    uint32_t l = std::max(last[ab[i].x], last[ab[i].y]) + 3u;
+    if (ab[i].x == end.x || ab[i].y == end.x || ab[i].x == end.y || ab[i].y == end.y) l = nb + 3u;
     if (l > i) lag = std::max(lag, l - i);
     if (lag > nb / 4) return;
   }
@@ -551,6 +549,36 @@ void split_chain(DBody& B, uint4* ab) {
   }
   B.sched = m;
   B.flags |= lag << BODY_LAG_SHIFT;
+}
+// Whether each half's consecutive links share exactly one particle; then the
+// records say which one is handed on (LINK_SWAPPED, LINK_KEEP).
+void carry_chain(DBody& B, uint4* ab) {
+  if (B.np > LINK_INDEX) return;
+  std::vector<uint32_t> on(B.nl);  // the endpoint that link k takes from the link before
+  auto has = [&](uint32_t k, uint32_t p) {
+    return (ab[k].x & LINK_INDEX) == p || (ab[k].y & LINK_INDEX) == p;
+  };
+  for (uint32_t half = 0; half < 2; ++half) {
+    const uint32_t k0 = half ? B.sched : 0u, k1 = half ? B.nl : B.sched;
+    for (uint32_t k = k0; k < k1; ++k) {
+      const uint32_t x = ab[k].x & LINK_INDEX, y = ab[k].y & LINK_INDEX;
+      if (k + 1 < k1) {
+        if (has(k + 1, x) == has(k + 1, y)) return;
+        on[k + 1] = has(k + 1, x) ? x : y;
+      }
+      if (k == k0) on[k] = k + 1 < k1 && on[k + 1] == x ? y : x;
+    }
+  }
+  for (uint32_t k = 0; k < B.nl; ++k) {
+    const bool end = k + 1 == B.nl || k + 1 == B.sched;
+    const bool keep = end || on[k + 1] == on[k];
+    if ((ab[k].x & LINK_INDEX) == on[k]) {
+      std::swap(ab[k].x, ab[k].y);
+      ab[k].x |= LINK_SWAPPED;
+    }
+    if (keep) ab[k].y |= LINK_KEEP;
+  }
+  B.flags |= BODY_CARRY;
 }
 }  // namespace
 
@@ -818,6 +846,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
         if (!(L.target_distance < 0x1p100f && L.target_distance > -0x1p100f)) B.flags &= ~BODY_RANGE;
       }
       split_chain(B, &im.lrec[B.l0]);
+      carry_chain(B, &im.lrec[B.l0]);
       im.serials.push_back((uint32_t)im.bodies.size());
       im.bodies.push_back(B);
       im.stats.serial_bodies++;
