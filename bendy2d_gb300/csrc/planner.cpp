@@ -132,6 +132,32 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
       d.tl = std::min(std::max((d.tl + 31u) & ~31u, 32u), 512u);
     }
     if (max_integ) d.ti = std::min((max_integ + 31u) & ~31u, max_link ? 256u : 512u);
+    if (max_link) {
+      // Fewer link threads where the shorter rounds outweigh the more of them:
+      // warps without an op issue a round's instructions too.  Measured on
+      // bodies of 840 to 4,200 particles, a round takes 0.11, 0.13, 0.15 or
+      // 0.19 us with one to four link warps on a scheduler, beside a time for
+      // each op.  41x27 in fast order (levels of 509 to 553 links): 512
+      // threads 486 rounds 126 us, 320 threads 519 rounds 111 us; 52x42: 512
+      // threads 208 us, 384 threads 189 us; but 36x30 (480 to 540 links): 512
+      // threads 353 rounds 101 us, 320 threads 519 rounds 109 us.
+      auto cost = [&](uint32_t tl) {
+        constexpr uint32_t ROUND[4] = {11, 13, 15, 19};
+        uint64_t r = 0;
+        for (uint32_t l = 1; l <= maxl; ++l) r += (nlink[l] + tl - 1) / tl;
+        return r * ROUND[(tl + 127u) / 128u - 1u];
+      };
+      const uint64_t now = cost(d.tl);
+      uint64_t least = now - now / 20u;  // only for a gain of 5 %
+      for (uint32_t tl = d.tl; tl > std::max(t.t_min, 32u);) {
+        tl -= 32u;
+        const uint64_t c = cost(tl);
+        if (c <= least) {
+          least = c;
+          d.tl = tl;
+        }
+      }
+    }
     if (d.tl + d.ti == 0) d.tl = 32;
   }
   // cut the level sequence into chunks of rounds (a level may span chunks)

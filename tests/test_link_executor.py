@@ -130,3 +130,12 @@ def test_more_bodies_than_multiprocessors(gpu):
     for collide in (0, 1):
         _check(_scene(bodies, collide), f"400 bodies, collide {collide}", steps=2,
                tuning={"pack_np": 1})
+
+
+@pytest.mark.parametrize("collide", [0, 1])
+@pytest.mark.parametrize("w,h,mode", [(36, 30, 1), (41, 27, 1), (44, 26, 1), (45, 33, 0), (52, 42, 1)])
+def test_levels_a_little_wider_than_the_threads(gpu, w, h, mode, collide):
+    """Levels of several rounds, with and without fewer threads for them."""
+    sc = _scene([_grid(w, h)], collide, sub_steps=2, link_iters=4, stiff=0.9)
+    sc.mode = mode
+    _check(sc, f"{w}x{h} mode {mode}", steps=1)
