@@ -49,6 +49,14 @@ bool PlanTuning::set(const std::string& k, double v) {
   return true;
 }
 
+// A round's time with tl <= 512 link threads, in 10 ns, beside a time for each
+// op (measured on bodies of 840 to 4,200 particles): one to four warps a
+// scheduler.
+static uint32_t round_cost(uint32_t tl) {
+  constexpr uint32_t ROUND[4] = {11, 13, 15, 19};
+  return ROUND[(tl + 127u) / 128u - 1u];
+}
+
 uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I,
                             bool full, bool group, const PlanTuning& t) {
   std::string key;
@@ -134,18 +142,15 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
     if (max_integ) d.ti = std::min((max_integ + 31u) & ~31u, max_link ? 256u : 512u);
     if (max_link) {
       // Fewer link threads where the shorter rounds outweigh the more of them:
-      // warps without an op issue a round's instructions too.  Measured on
-      // bodies of 840 to 4,200 particles, a round takes 0.11, 0.13, 0.15 or
-      // 0.19 us with one to four link warps on a scheduler, beside a time for
-      // each op.  41x27 in fast order (levels of 509 to 553 links): 512
+      // warps without an op issue a round's instructions too (round_cost).
+      // 41x27 in fast order (levels of 509 to 553 links): 512
       // threads 486 rounds 126 us, 320 threads 519 rounds 111 us; 52x42: 512
       // threads 208 us, 384 threads 189 us; but 36x30 (480 to 540 links): 512
       // threads 353 rounds 101 us, 320 threads 519 rounds 109 us.
       auto cost = [&](uint32_t tl) {
-        constexpr uint32_t ROUND[4] = {11, 13, 15, 19};
         uint64_t r = 0;
         for (uint32_t l = 1; l <= maxl; ++l) r += (nlink[l] + tl - 1) / tl;
-        return r * ROUND[(tl + 127u) / 128u - 1u];
+        return r * round_cost(tl);
       };
       const uint64_t now = cost(d.tl);
       uint64_t least = now - now / 20u;  // only for a gain of 5 %
@@ -324,8 +329,25 @@ uint32_t SchedRegistry::get_flow(const uint2* links, uint32_t nl, uint32_t np, u
   DSched d{};
   d.nlvl = nlvl;
   d.nops = (uint32_t)seq.size();
-  d.tl = std::min(std::max((max_link + 31u) & ~31u, 32u), 512u);
   d.ti = max_integ ? std::min((max_integ + 31u) & ~31u, 256u) : 0u;
+  // Link threads as in get(), over the widest CTA of each level: 100x100 over
+  // seven CTAs has 576 to 616 links in the widest one on 445 of 685 levels: two
+  // rounds of 512 threads 526 us an update, one of 640 519 us, two of 320
+  // 495 us.
+  d.tl = std::min(std::max((max_link + 31u) & ~31u, 32u), 512u);
+  std::vector<uint32_t> widest(nlvl, 0);
+  for (uint32_t r = 0; r < C; ++r)
+    for (uint32_t l = 0; l < nlvl; ++l) {
+      const size_t g = (size_t)r * nlvl + l;
+      widest[l] = std::max(widest[l], count[3 * g + 2] - count[3 * g]);
+    }
+  auto cost = [&](uint32_t tl) {
+    uint64_t n = 0;
+    for (uint32_t w : widest) n += (w + tl - 1) / tl;
+    return n * round_cost(tl);
+  };
+  for (uint32_t tl = d.tl; tl >= 32u; tl -= 32u)
+    if (cost(tl) < cost(d.tl)) d.tl = tl;
   d.chunk0 = (uint32_t)chunk_off.size();
   std::vector<uint32_t> rec((size_t)C * FLOW_REC_WORDS, 0);
   for (uint32_t r = 0; r < C; ++r) {
@@ -842,7 +864,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // Serial or by levels: a body whose single pass is narrow may still be wide
     // over the passes its schedule chains, which start behind one another.
     // Measured on 24 ropes of 200 particles (one pass 1 wide, the 8 x 4 passes
-    // of an update ~29): 1,710 us a pass replayed by one thread each, 79 us by
+    // of an update ~29): 1,710 us a pass replayed by one thread each, 60 us by
     // levels.  Rings of a hub and spokes stay below 3 (the next pass's rim
     // runs beside this pass's spokes) and run serially.
     const PassDepth pd = pass_depth(w, c, tune.serial_width, last);

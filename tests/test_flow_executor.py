@@ -88,3 +88,11 @@ def test_more_clusters_than_the_gpu_holds(gpu):
     bodies = [_cloth(24 + k % 3, 20, (5.0 + 28.0 * (k % 10), 5.0 + 25.0 * (k // 10)), seed=k)
               for k in range(80)]
     _check(_scene(bodies), "80 bodies", tuning={"smem_max": 1024, "pack_np": 1})
+
+
+@pytest.mark.parametrize("w,h,mode", [(100, 100, 0), (72, 80, 1)])
+def test_levels_of_more_links_than_threads(gpu, w, h, mode):
+    """The widest CTA's levels take two rounds of fewer threads."""
+    sc = _scene([_cloth(w, h)], sub_steps=2, link_iters=4)
+    sc.mode = mode
+    _check(sc, f"{w}x{h} mode {mode}", steps=1)
