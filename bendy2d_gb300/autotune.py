@@ -4,10 +4,12 @@ Coordinate descent from the defaults: for one tunable at a time, each
 candidate value is timed on the real scene (CUDA events around `steps`
 updates after warm-up) and the fastest kept.  Tunables:
 
-  width_per_thread  group size T = pow2 >= (mean level width / this)
-  t_max             largest group size
+  width_per_thread  a group's link threads: those of its widest level, at most
+                    pow2 >= (mean level width / this)
+  t_max             most link threads of a group
   max_groups        groups per CTA for T > 32 (1 spreads bodies over SMs)
-  serial_width      schedule width below which a body runs serially
+  serial_width      width of one pass below which a body runs serially (and
+                    1.5 x this over all the passes of its schedule)
   resident          hold a body's whole schedule in shared memory when it fits
   stage_frac        serial bodies with chains >= this x the longest run alone,
                     links staged in shared memory

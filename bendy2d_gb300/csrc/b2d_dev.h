@@ -190,7 +190,7 @@ struct DWorld {
   float2* pcenter;
   float4* paabb;
   uint2* plab; float* plrest;
-  uint32_t* stage_off;   // polygon-pair test offsets, see rigid_phase_a
+  uint32_t* stage_off;   // polygon-pair test offsets, see stage_pair
   uint32_t* stage_pr;    // polygon pair of each stage: self | other << 16
 };
 

@@ -31,24 +31,23 @@ enum : int { FAULT_WAIT_TIMEOUT = 1, FAULT_GRID_CAP = 2, FAULT_ALLOC = 3 };
 struct PlanTuning {
   float serial_width = 2.0f;        // a body narrower than this in one pass, and than 1.5 x this
                                     // over all the passes of its schedule, runs serially
-  uint32_t t_min = 32, t_max = 512; // threads per group
+  uint32_t t_min = 32, t_max = 512; // link threads per group
   uint32_t pack_np = 1024;          // pack small components into bodies up to this size
   uint32_t pack_nl = 4096;
   uint32_t free_chunk = 2048;       // particles per body for link-free particles
   uint32_t smem_max = 200 * 1024;   // bytes of shared memory per group region
   uint32_t warp_groups = 8;         // groups per CTA when T == 32
   uint32_t max_groups = 15;         // groups per CTA when T > 32
-  float width_per_thread = 0.5f;    // T = pow2 >= avg width / this (issue-bound: wide groups win)
+  float width_per_thread = 0.5f;    // link threads: at most pow2 >= avg width / this
   uint32_t resident = 1;            // load a body's whole schedule when it fits
   uint32_t res_max = 227 * 1024;    // shared bytes per group for body + resident schedule
   float stage_frac = 1.01f;         // serial bodies with chains >= this x the longest: solo
-                                    // packs, links staged in shared memory (default: none;
-                                    // with positions forwarded in registers ordinary packs
-                                    // run the longest chains faster)
+                                    // packs, links staged in shared memory (default: none,
+                                    // as ordinary packs run the longest chains faster cold)
   float bucket_factor = 2.0f;       // collision-grid buckets per world: pow2 >= this x particles
   uint32_t collide_thread_min = 81920;  // particles in the collide pass from which it runs
                                          // one thread per particle (else three lanes each)
-  uint32_t large_max = 8;           // largest cluster of the large-body executor (0: bodies
+  uint32_t large_max = 8;           // largest cluster of the flow and large executors (0: bodies
                                     // over one CTA's shared memory run from global memory)
   uint32_t grid_slot_max = 262144;  // particles in the collision grid up to which it is
                                     // built by slot inserts; above, by a counting sort per
@@ -91,7 +90,7 @@ struct GroupBody {
 
 struct PlanStats {
   uint32_t bodies = 0, group_bodies = 0, serial_bodies = 0, global_bodies = 0;
-  uint32_t large_bodies = 0;  // group bodies run by the large-body executor
+  uint32_t large_bodies = 0;  // group bodies run by the flow or large executor
   uint64_t levels = 0, ops = 0;  // summed over group bodies
   uint32_t colours = 0;
 };

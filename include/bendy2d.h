@@ -179,9 +179,9 @@ typedef struct {
   uint64_t levels, ops;
   uint32_t colours;
   uint64_t device_bytes;
-  /* group bodies over one CTA's shared memory that the large-body executor
-   * runs from the shared memory of a thread-block cluster (global_bodies
-   * counts the ones run from global memory) */
+  /* group bodies over one CTA's shared memory that run from the shared memory
+   * of a thread-block cluster (global_bodies counts the ones run from global
+   * memory) */
   uint32_t large_bodies;
 } b2d_plan_stats;
 int b2d_get_plan_stats(b2d_solver* s, b2d_plan_stats* out);
