@@ -63,10 +63,12 @@ constexpr uint32_t LINK_SWAPPED = 0x40000000u, LINK_KEEP = 0x40000000u;
 constexpr uint32_t LINK_INDEX = 0x3FFFFFFFu;
 constexpr uint32_t NO_FIRST = 0xFFFFFFFFu;
 
-// a serial record's endpoints in the link's order
-__host__ __device__ inline uint2 record_ends(const uint4& r) {
-  const uint32_t x = r.x & LINK_INDEX, y = r.y & LINK_INDEX;
-  return (r.x & LINK_SWAPPED) ? uint2{y, x} : uint2{x, y};
+// a serial record's endpoints in the link's order (carried: its body is one of
+// BODY_CARRY; others may index past LINK_INDEX)
+__host__ __device__ inline uint2 record_ends(const uint4& r, bool carried) {
+  const uint32_t mask = carried ? LINK_INDEX : ~LINK_FINAL;
+  const uint32_t x = r.x & mask, y = r.y & mask;
+  return carried && (r.x & LINK_SWAPPED) ? uint2{y, x} : uint2{x, y};
 }
 
 struct DPoly {

@@ -463,7 +463,7 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
       return bad("body first particle");
     const uint32_t lim = B.local ? B.np : P.np;
     for (uint32_t k = 0; k < B.nl; ++k) {
-      const uint2 e = serial ? record_ends(im.lrec[B.l0 + k]) : im.lab[B.l0 + k];
+      const uint2 e = serial ? record_ends(im.lrec[B.l0 + k], B.flags & BODY_CARRY) : im.lab[B.l0 + k];
       if (e.x >= lim || e.y >= lim || e.x == e.y) return bad("link endpoint");
     }
   }
