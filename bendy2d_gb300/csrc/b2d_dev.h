@@ -101,6 +101,12 @@ constexpr uint32_t sched_head_words(uint32_t n) { return (n + 4u) & ~1u; }
 // shared bytes after each executor group's schedule area: two mbarriers and
 // two flag words
 constexpr uint32_t GROUP_TAIL_BYTES = 32;
+// Threads of a group executor's CTA, one group or several: at most 512 link
+// and 256 integrate threads in a whole update; a link pass, whose launches may
+// have more bodies than SMs, stays within the 64 registers that let two CTAs
+// of 512 threads share an SM (200 cloths of 32x32, a pass: 44 us; with 70
+// registers 61 us).
+constexpr uint32_t group_threads_max(bool full) { return full ? 768u : 512u; }
 struct DSched {
   uint32_t chunk0, nchunks;  // chunk_off / chunk_len entries
   uint32_t nlvl, nops;

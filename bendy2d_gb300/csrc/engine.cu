@@ -802,7 +802,7 @@ int Engine::rebuild_lists() {
     uint32_t G = c.T == 32 ? tune_.warp_groups : std::max<uint32_t>(1, 256 / c.T);
     if (c.T != 32) G = std::min<uint32_t>(G, std::min<uint32_t>(tune_.max_groups, 15));
     G = c.skip ? std::max<uint32_t>(G, 1) : 1;
-    G = std::min<uint32_t>(G, std::max<uint32_t>(1, GROUP_THREADS_MAX / c.T));
+    G = std::min<uint32_t>(G, std::max<uint32_t>(1, group_threads_max(c.full) / c.T));
     c.G = std::max<uint32_t>(1, std::min<uint32_t>(G, (uint32_t)g_smem_optin / per_group));
   }
   if (!plain_) build_packs(sfull_all, true, packs_full_, serial_full_, true);

@@ -500,7 +500,8 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
       return bad("large-body executor layout");
     if (g.res && (!g.smem || g.res != S.words * 4u)) return bad("resident schedule size");
     if (g.T < 32 || g.T % 32) return bad("group size");
-    if (g.smem && (S.tl + S.ti != g.T || S.tl % 32 || S.tl > 512u || S.ti > 512u || g.T > 768u)) return bad("group threads");
+    if (g.smem && (S.tl + S.ti != g.T || S.tl % 32)) return bad("group threads");
+    if (!g.large_c && g.T > group_threads_max(!im.ext)) return bad("group threads");
   }
   for (uint32_t b : im.serials) {
     if (b >= im.bodies.size() || !im.bodies[b].local || !(im.bodies[b].flags & BODY_SERIAL))
@@ -797,7 +798,7 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     const DSched& S = reg.scheds[B.sched];
     const float avg = S.nlvl ? (float)S.nops / (float)S.nlvl : 1.0f;
     uint32_t T = pow2ceil((uint32_t)(avg / tune.width_per_thread + 0.999f));
-    T = std::min(std::max(T, tune.t_min), tune.t_max);
+    T = std::min(std::min(std::max(T, tune.t_min), tune.t_max), group_threads_max(full));
     if (smem || flow_c) T = S.tl + S.ti;
     // the whole schedule resident in shared memory when it fits beside the body
     uint32_t res = 0;
