@@ -12,6 +12,7 @@
 // run ahead into later passes (the critical path of a 32x32 cloth step drops
 // from 4032 to ~413 levels).
 #include <algorithm>
+#include <array>
 #include <cstdlib>
 #include <cstring>
 #include <numeric>
@@ -241,6 +242,44 @@ uint32_t SchedRegistry::get(const uint2* links, uint32_t nl, uint32_t np, uint32
   return id;
 }
 
+// CTA r of a flow body integrates particles [np*r/C, np*(r+1)/C) and solves the
+// links whose first endpoint is one of them.
+static void flow_owners(uint32_t np, uint32_t C, std::vector<uint32_t>& own, std::vector<uint8_t>& cta) {
+  own.resize(C + 1);
+  for (uint32_t r = 0; r <= C; ++r) own[r] = (uint32_t)((uint64_t)np * r / C);
+  cta.resize(np);
+  for (uint32_t r = 0; r < C; ++r)
+    for (uint32_t p = own[r]; p < own[r + 1]; ++p) cta[p] = (uint8_t)r;
+}
+
+// The most of a CTA's {window, own particles, links} in the flow schedule over
+// C CTAs, known before any of it is built.
+static std::array<uint32_t, 3> flow_sizes(const uint2* links, uint32_t nl, uint32_t np, bool solves,
+                                          bool integrates, uint32_t C) {
+  std::vector<uint32_t> own;
+  std::vector<uint8_t> cta;
+  flow_owners(np, C, own, cta);
+  std::vector<uint32_t> lo(own.begin(), own.end() - 1), hi(lo), count(C, 0);
+  for (uint32_t r = 0; r < C; ++r) {
+    if (integrates) hi[r] = own[r + 1];
+    else if (solves) lo[r] = np;  // its links' particles alone
+  }
+  for (uint32_t k = 0; k < nl; ++k) {
+    const uint32_t r = cta[links[k].x];
+    ++count[r];
+    if (!solves) continue;
+    lo[r] = std::min(lo[r], std::min(links[k].x, links[k].y));
+    hi[r] = std::max(hi[r], std::max(links[k].x, links[k].y) + 1);
+  }
+  std::array<uint32_t, 3> most{1, 0, 0};
+  for (uint32_t r = 0; r < C; ++r) {
+    if (hi[r] > lo[r]) most[0] = std::max(most[0], hi[r] - lo[r]);
+    most[1] = std::max(most[1], own[r + 1] - own[r]);
+    most[2] = std::max(most[2], count[r]);
+  }
+  return most;
+}
+
 uint32_t SchedRegistry::get_flow(const uint2* links, uint32_t nl, uint32_t np, uint32_t S, uint32_t I,
                                  bool full, uint32_t C) {
   std::string key;
@@ -252,13 +291,9 @@ uint32_t SchedRegistry::get_flow(const uint2* links, uint32_t nl, uint32_t np, u
   if (it != index.end()) return it->second;
   if (np > 65535u || C < 2 || C > FLOW_MAX_C || np < C) return NONE;
 
-  // CTA r integrates particles [np*r/C, np*(r+1)/C) and solves the links
-  // whose first endpoint is one of them
-  std::vector<uint32_t> own(C + 1);
-  for (uint32_t r = 0; r <= C; ++r) own[r] = (uint32_t)((uint64_t)np * r / C);
-  std::vector<uint8_t> cta(np);
-  for (uint32_t r = 0; r < C; ++r)
-    for (uint32_t p = own[r]; p < own[r + 1]; ++p) cta[p] = (uint8_t)r;
+  std::vector<uint32_t> own;
+  std::vector<uint8_t> cta;
+  flow_owners(np, C, own, cta);
   std::vector<uint32_t> lidx(nl);  // link -> its index among its CTA's links
   std::vector<std::vector<uint32_t>> mine(C);
   for (uint32_t k = 0; k < nl; ++k) {
@@ -485,7 +520,8 @@ static bool check_image(const WorldImage& im, const SchedRegistry& reg, std::str
         const uint32_t* R = &reg.stream[S.off + r * FLOW_REC_WORDS];
         if ((size_t)R[FR_CHUNK0] + R[FR_NCHUNKS] > reg.chunk_off.size() ||
             R[FR_LO] + R[FR_WINDOW] > B.np || 8u * R[FR_WINDOW] > g.flow_pos || R[FR_OWN1] > B.np ||
-            R[FR_NLEVELS] != S.nlvl)
+            (!im.ext && 8u * (R[FR_OWN1] - R[FR_OWN0]) > g.flow_prev) ||
+            (B.flags & BODY_UNIT ? 4u : 8u) * R[FR_NLINKS] > g.flow_rest || R[FR_NLEVELS] != S.nlvl)
           return bad("flow executor record");
         for (uint32_t f : {FR_LINKS, FR_LOAD, FR_STORE, FR_EXPECT})
           if ((size_t)R[f] + R[f + 1] > reg.stream.size()) return bad("flow executor list");
@@ -775,22 +811,20 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
       uint32_t c = (uint32_t)std::min(std::max(wide / 400.0, 2.0), (double)FLOW_MAX_C);
       const uint32_t most = std::min(tune.large_max, FLOW_MAX_C);
       for (c = std::min(c, most); c <= most && !flow_c; ++c) {
-        // (what it takes at the least, before its schedule is built)
-        const size_t least = (state + (B.flags & BODY_UNIT ? 4u : 8u) * (size_t)B.nl) / c;
+        // (what it takes at the least, and then exactly, before its schedule
+        // is built: only the one that is used is kept and uploaded)
+        const uint32_t per_link = B.flags & BODY_UNIT ? 4u : 8u;
+        const size_t least = (state + per_link * (size_t)B.nl) / c;
         if (least + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
+        const auto most_of = flow_sizes(loc.data(), B.nl, B.np, P.I > 0 && (!full || P.S > 0),
+                                        full && P.S > 0, c);
+        const size_t need[3] = {align16(8 * (size_t)most_of[0]), full ? align16(8 * (size_t)most_of[1]) : 0,
+                                align16(per_link * (size_t)most_of[2])};
+        if (need[0] + need[1] + need[2] + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
         const uint32_t id = reg.get_flow(loc.data(), B.nl, B.np, P.S, P.I, full, c);
         if (id == SchedRegistry::NONE) break;
-        uint32_t need[3] = {0, 0, 0};
-        for (uint32_t r = 0; r < c; ++r) {
-          const uint32_t* R = &reg.stream[reg.scheds[id].off + r * FLOW_REC_WORDS];
-          need[0] = std::max(need[0], 8u * R[FR_WINDOW]);
-          if (full) need[1] = std::max(need[1], 8u * (R[FR_OWN1] - R[FR_OWN0]));
-          need[2] = std::max(need[2], (B.flags & BODY_UNIT ? 4u : 8u) * R[FR_NLINKS]);
-        }
-        for (uint32_t& v : need) v = (uint32_t)align16(v);
-        if ((size_t)need[0] + need[1] + need[2] + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
         flow_c = c;
-        std::copy(need, need + 3, flow);
+        for (int k = 0; k < 3; ++k) flow[k] = (uint32_t)need[k];
         B.sched = id;
       }
     }
