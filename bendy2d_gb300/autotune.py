@@ -9,7 +9,8 @@ updates after warm-up) and the fastest kept.  Tunables:
   t_max             most link threads of a group
   max_groups        groups per CTA for T > 32 (1 spreads bodies over SMs)
   serial_width      width of one pass below which a body runs serially (and
-                    1.5 x this over all the passes of its schedule)
+                    1.5 x this over all the passes of its schedule, or 3.5 x
+                    for chains that the large-body executor would run)
   resident          hold a body's whole schedule in shared memory when it fits
   stage_frac        serial bodies with chains >= this x the longest run alone,
                     links staged in shared memory

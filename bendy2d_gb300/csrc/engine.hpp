@@ -30,7 +30,8 @@ enum : int { FAULT_WAIT_TIMEOUT = 1, FAULT_GRID_CAP = 2, FAULT_ALLOC = 3 };
 // Tunables of the planner (the autotuner sweeps these).
 struct PlanTuning {
   float serial_width = 2.0f;        // a body narrower than this in one pass, and than 1.5 x this
-                                    // over all the passes of its schedule, runs serially
+                                    // over all the passes of its schedule (3.5 x where the
+                                    // large-body executor would run it), runs serially
   uint32_t t_min = 32, t_max = 512; // link threads per group
   uint32_t pack_np = 1024;          // pack small components into bodies up to this size
   uint32_t pack_nl = 4096;

@@ -749,6 +749,61 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
   std::vector<const Comp*> pack;
   uint32_t pack_np = 0, pack_nl = 0;
 
+  // The executor of a group body, chosen by its size with stiffness (a body of
+  // unit stiffness takes less): one CTA's shared memory; over that the flow
+  // executor, over as many CTAs as give each ~200 ops a level, at least as many
+  // as hold it; failing that (more than 65,535 particles, or too much for
+  // large_max CTAs) the large-body executor, which keeps its positions (and
+  // prev) in the shared memory of a cluster of up to large_max CTAs, at most
+  // 128 KB each (8,192 particles whole-step, 16,384 for link passes), with link
+  // parameters and schedule read through the caches; beyond that the group
+  // executor from global memory.
+  struct Place {
+    bool smem;
+    uint32_t flow_c, flow[3];    // CTAs; bytes of positions, prev and link parameters in each
+    uint32_t large_c, log2per;
+  };
+  auto fits_cta = [&](size_t n, size_t links) {
+    return align16((full ? 16u : 8u) * n + 8u * links) <= tune.smem_max && n <= 65535u;
+  };
+  auto place = [&](const uint2* loc, uint32_t n, uint32_t links, bool unit, uint32_t pass_levels) {
+    Place at{};
+    const size_t state = (full ? 16u : 8u) * (size_t)n;
+    at.smem = fits_cta(n, links);
+    if (at.smem) return at;
+    if (tune.large_max >= 2 && n <= 65535u) {
+      const double wide = (double)links / std::max((double)pass_levels, 1.0) *
+                          (full ? (double)P.S * P.I : P.I);
+      const uint32_t most = std::min(tune.large_max, FLOW_MAX_C);
+      uint32_t c = (uint32_t)std::min(std::max(wide / 400.0, 2.0), (double)FLOW_MAX_C);
+      for (c = std::min(c, most); c <= most && c <= n; ++c) {
+        // (what it takes at the least, and then exactly)
+        const uint32_t per_link = unit ? 4u : 8u;
+        const size_t least = (state + per_link * (size_t)links) / c;
+        if (least + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
+        const auto most_of = flow_sizes(loc, links, n, P.I > 0 && (!full || P.S > 0),
+                                        full && P.S > 0, c);
+        const size_t need[3] = {align16(8 * (size_t)most_of[0]), full ? align16(8 * (size_t)most_of[1]) : 0,
+                                align16(per_link * (size_t)most_of[2])};
+        if (need[0] + need[1] + need[2] + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
+        at.flow_c = c;
+        for (int k = 0; k < 3; ++k) at.flow[k] = (uint32_t)need[k];
+        return at;
+      }
+    }
+    if (tune.large_max > 0 && n > 0) {
+      const uint32_t cap_log2 = full ? 13u : 14u;
+      uint32_t l2 = 0;
+      while (l2 < cap_log2 && (1u << l2) < n) ++l2;
+      const uint32_t c = (n + (1u << l2) - 1u) >> l2;
+      if (c <= tune.large_max) {
+        at.large_c = c;
+        at.log2per = l2;
+      }
+    }
+    return at;
+  };
+
   struct Item { uint2 e; float rest, stiff; uint32_t level; };
   std::vector<Item> seq;                // emit_group's, kept between bodies
   std::vector<uint32_t> depth, at;
@@ -794,46 +849,18 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
       if (it.stiff != 1.0f) B.flags &= ~BODY_UNIT;
       if (!(it.rest < 0x1p100f && it.rest > -0x1p100f)) B.flags &= ~BODY_RANGE;
     }
-    // the executor is chosen by the body's size with stiffness; a body of
-    // unit stiffness takes less
-    const size_t state = (full ? 16u : 8u) * (size_t)B.np;
-    const bool smem = align16(state + 8u * (size_t)B.nl) <= tune.smem_max && B.np <= 65535u;
-    const size_t region = align16(state + (B.flags & BODY_UNIT ? 4u : 8u) * (size_t)B.nl);
-    // A body over one CTA's shared memory: the flow executor, over as many CTAs
-    // as give each ~200 ops a level, at least as many as hold it; failing that
-    // (more than 65,535 particles, or too much for large_max CTAs) the
-    // large-body executor below, and beyond it the group executor from
-    // global memory.
-    uint32_t flow_c = 0, flow[3] = {0, 0, 0};
-    if (!smem && tune.large_max >= 2 && B.np <= 65535u) {
-      const double depth_est = (double)at.size() - 1.0;  // levels of one pass
-      const double wide = (double)B.nl / std::max(depth_est, 1.0) * (full ? (double)P.S * P.I : P.I);
-      uint32_t c = (uint32_t)std::min(std::max(wide / 400.0, 2.0), (double)FLOW_MAX_C);
-      const uint32_t most = std::min(tune.large_max, FLOW_MAX_C);
-      for (c = std::min(c, most); c <= most && !flow_c; ++c) {
-        // (what it takes at the least, and then exactly, before its schedule
-        // is built: only the one that is used is kept and uploaded)
-        const uint32_t per_link = B.flags & BODY_UNIT ? 4u : 8u;
-        const size_t least = (state + per_link * (size_t)B.nl) / c;
-        if (least + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
-        const auto most_of = flow_sizes(loc.data(), B.nl, B.np, P.I > 0 && (!full || P.S > 0),
-                                        full && P.S > 0, c);
-        const size_t need[3] = {align16(8 * (size_t)most_of[0]), full ? align16(8 * (size_t)most_of[1]) : 0,
-                                align16(per_link * (size_t)most_of[2])};
-        if (need[0] + need[1] + need[2] + FLOW_TAIL_BYTES + STREAM_BUFFERS > tune.res_max) continue;
-        const uint32_t id = reg.get_flow(loc.data(), B.nl, B.np, P.S, P.I, full, c);
-        if (id == SchedRegistry::NONE) break;
-        flow_c = c;
-        for (int k = 0; k < 3; ++k) flow[k] = (uint32_t)need[k];
-        B.sched = id;
-      }
-    }
-    if (!flow_c) B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, smem, tune);
+    const bool unit = (B.flags & BODY_UNIT) != 0u;
+    const Place pl = place(loc.data(), B.np, B.nl, unit, (uint32_t)at.size() - 1u);
+    const bool smem = pl.smem;
+    const size_t region = align16((full ? 16u : 8u) * (size_t)B.np + (unit ? 4u : 8u) * (size_t)B.nl);
+    if (pl.flow_c) B.sched = reg.get_flow(loc.data(), B.nl, B.np, P.S, P.I, full, pl.flow_c);
+    else B.sched = reg.get(loc.data(), B.nl, B.np, P.S, P.I, full, smem, tune);
+    if (B.sched == SchedRegistry::NONE) std::abort();  // place() chose what a schedule can hold
     const DSched& S = reg.scheds[B.sched];
     const float avg = S.nlvl ? (float)S.nops / (float)S.nlvl : 1.0f;
     uint32_t T = pow2ceil((uint32_t)(avg / tune.width_per_thread + 0.999f));
     T = std::min(std::min(std::max(T, tune.t_min), tune.t_max), group_threads_max(full));
-    if (smem || flow_c) T = S.tl + S.ti;
+    if (smem || pl.flow_c) T = S.tl + S.ti;
     // the whole schedule resident in shared memory when it fits beside the body
     uint32_t res = 0;
     if (smem && tune.resident) {
@@ -841,27 +868,12 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
       if (region + sb + GROUP_TAIL_BYTES <= tune.res_max)
         res = (uint32_t)sb;
     }
-    // A body over one CTA's shared memory: the large-body executor keeps its
-    // positions (and prev) in the shared memory of a cluster of up to
-    // large_max CTAs, at most 128 KB each (8,192 particles whole-step,
-    // 16,384 for link passes), with link parameters and schedule read
-    // through the caches; beyond that the group executor runs it from
-    // global memory.
-    uint32_t large_c = 0, log2per = 0, TL = T;
-    if (!smem && !flow_c && tune.large_max > 0 && B.np > 0) {
-      const uint32_t cap_log2 = full ? 13u : 14u;
-      uint32_t l2 = 0;
-      while (l2 < cap_log2 && (1u << l2) < B.np) ++l2;
-      const uint32_t c = (B.np + (1u << l2) - 1u) >> l2;
-      if (c <= tune.large_max) {
-        large_c = c;
-        log2per = l2;
-        const float w = avg / (tune.width_per_thread * (float)c);
-        TL = std::min<uint32_t>(1024u, std::max<uint32_t>(64u, pow2ceil((uint32_t)(w + 0.999f))));
-      }
-    }
-    if (flow_c) {
-      large_c = flow_c;
+    uint32_t large_c = pl.large_c, TL = T;
+    if (large_c) {
+      const float w = avg / (tune.width_per_thread * (float)large_c);
+      TL = std::min<uint32_t>(1024u, std::max<uint32_t>(64u, pow2ceil((uint32_t)(w + 0.999f))));
+    } else if (pl.flow_c) {
+      large_c = pl.flow_c;
       TL = T + 32;  // and the control warp
     }
     const bool local = smem || large_c > 0;
@@ -874,10 +886,10 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     im.bodies.push_back(B);
     GroupBody gbody{id, large_c ? TL : T, smem ? (uint32_t)region : 0u, res, smem};
     gbody.large_c = large_c;
-    gbody.log2per = log2per;
-    gbody.flow_pos = flow[0];
-    gbody.flow_prev = flow[1];
-    gbody.flow_rest = flow[2];
+    gbody.log2per = pl.log2per;
+    gbody.flow_pos = pl.flow[0];
+    gbody.flow_prev = pl.flow[1];
+    gbody.flow_rest = pl.flow[2];
     im.groups.push_back(gbody);
     im.stats.group_bodies++;
     if (large_c) im.stats.large_bodies++;
@@ -891,6 +903,21 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     pack_np = pack_nl = 0;
   };
 
+  // whether the large-body executor would run a component by levels
+  auto to_large = [&](const Comp& c, uint32_t pass_levels) {
+    if (fits_cta(c.parts.size(), c.links.size())) return false;
+    std::vector<uint2> loc;
+    loc.reserve(c.links.size());
+    for (size_t i = 0; i < c.parts.size(); ++i) local[c.parts[i]] = (uint32_t)i;
+    bool unit = true;
+    for (uint32_t k : c.links) {
+      const Link& L = w.particle_links[k];
+      loc.push_back(make_uint2(local[L.particle_a], local[L.particle_b]));
+      unit &= L.stiffness == 1.0f;
+    }
+    return place(loc.data(), (uint32_t)c.parts.size(), (uint32_t)loc.size(), unit, pass_levels).large_c != 0u;
+  };
+
   for (const Comp& c : comps) {
     if (c.links.empty()) {
       free_parts.push_back(c.parts[0]);
@@ -901,13 +928,23 @@ int plan_world(const WorldHost& w, const PlanTuning& tune, SchedRegistry& reg, W
     // Measured on 24 ropes of 200 particles (one pass 1 wide, the 8 x 4 passes
     // of an update ~29): 1,710 us a pass replayed by one thread each, 60 us by
     // levels.  Rings of a hub and spokes stay below 3 (the next pass's rim
-    // runs beside this pass's spokes) and run serially.
+    // runs beside this pass's spokes) and run serially.  3 is near the crossing
+    // on every executor but one (2 x 1 passes, width 4, serially and by levels:
+    // ropes of 11,000 and 30,000 on the flow executor 6.8 and 3.4 ms, 19.8 and
+    // 9.3; of 70,000 from global memory 45.9 and 39.5): a level of the
+    // large-body executor costs 1.1 us, and in its link passes a rope of 70,000
+    // takes 52.7 ms serially and 79.6 by levels at width 4, 79.2 and 79.8 at 6,
+    // 105.7 and 79.9 at 8, one with braces 144.6 and 159.9 at 6, 192.9 and
+    // 160.6 at 8.  So it takes chains from 7.
     const PassDepth pd = pass_depth(w, c, tune.serial_width, last);
     const double passes = full ? (double)P.S * P.I : (double)P.I;
     const double ops = passes * (double)c.links.size() + (full ? (double)P.S * c.parts.size() : 0.0);
     const double levels = (double)pd.first + (passes - 1.0) * pd.more + (full ? (double)P.S : 0.0);
     const double width = (double)c.links.size() / (double)std::max(pd.first, 1u);
-    if (width < tune.serial_width && ops / std::max(levels, 1.0) < 1.5 * tune.serial_width) {
+    const double many = ops / std::max(levels, 1.0);
+    if (width < tune.serial_width &&
+        (many < 1.5 * tune.serial_width ||
+         (many < 3.5 * tune.serial_width && to_large(c, pd.first)))) {
       DBody B{};
       B.i0 = (uint32_t)im.bidx.size();
       B.np = (uint32_t)c.parts.size();
