@@ -143,6 +143,7 @@ struct LaunchClass {
   uint32_t words;  // largest member schedule, in words
   bool smem, full;
   bool skip = false;  // more bodies than SMs: idle warps skip a round's work
+  bool free = false;  // wide bodies without link ops: any number of threads runs them
   uint32_t large_c = 0, log2per = 0;  // large-body executor class (large_c CTAs per body)
   uint32_t flow_pos = 0, flow_prev = 0, flow_rest = 0;  // flow executor class: its bodies'
   std::vector<uint2> items;
