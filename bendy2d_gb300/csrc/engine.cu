@@ -1182,13 +1182,13 @@ int Engine::launch_all(bool profiling) {
       auto collide = [&](const auto& grid, auto rigid) {
         using GRID = std::decay_t<decltype(grid)>;
         constexpr bool RIGID = decltype(rigid)::value;
-        const uint32_t nct = nch * COLLIDE_CTAS;
+        const uint32_t nct = nch * COLLIDE_CTAS, sms = (uint32_t)std::max(g_num_sms, 1);
         if (collide_per_particle_)
           lk(launch_k(k_collide_particle<GRID, RIGID>, dim3(nch), dim3(COLLIDE_P_THREADS), 0, stream_,
                       !profiling, W, grid, CH, nch, cur, s));
-        else  // six CTAs an SM where five would leave a few for a second wave
-          lk(launch_k(nct <= 5u * (uint32_t)std::max(g_num_sms, 1) ? k_collide_integrate<GRID, 5, RIGID>
-                                                                 : k_collide_integrate<GRID, 6, RIGID>,
+        else  // six CTAs an SM where they make one wave and five would leave a few for a second
+          lk(launch_k(nct > 5u * sms && nct <= 6u * sms ? k_collide_integrate<GRID, 6, RIGID>
+                                                        : k_collide_integrate<GRID, 5, RIGID>,
                       dim3(nct), dim3(COLLIDE_THREADS), 0, stream_, !profiling, W, grid, CH, nch,
                       cur, s));
       };
