@@ -534,8 +534,9 @@ def kernel_rooflines(prof: dict, sc, launches_per_step: dict) -> dict:
 
 # Warp-instructions per link solve of the shared-memory link executor, from
 # its ncu captures (instructions executed / link solves of the launch):
-# configuration 5 (fast order), 98.4 M / 32.0 M; configuration 2, 3.62 M / 1.0 M.
-LINK_WARP_INSTR = {"config5": 98.43e6 / (1024 * 3906 * 8), "config2": 3.616e6 / (64 * 3906 * 4)}
+# configuration 5 (fast order), 98.4 M / 32.0 M (profiles/config5_collide_and_links.md);
+# configuration 2, 3.62 M / 1.0 M (profiles/exec_groups_links_config2.md).
+LINK_WARP_INSTR = {"config5": 98.45e6 / (1024 * 3906 * 8), "config2": 3.616e6 / (64 * 3906 * 4)}
 
 
 def link_issue_bound(torch, ms_per_step: float, solves_per_step: float, per_solve: float) -> dict:

@@ -797,7 +797,7 @@ int Engine::rebuild_lists() {
     // streamed: one 16 KB chunk per fill, or for launches with no more bodies
     // than SMs (latency-bound) the largest fills that fit beside the body,
     // which cuts the buffer switches of long schedules
-    c.fill = STREAM_BUF_BYTES / 2;
+    c.fill = STREAM_BUFFERS / 2;
     if (!c.res && c.items.size() <= (size_t)std::max(g_num_sms, 1)) {
       const uint32_t room = ((uint32_t)g_smem_optin - c.region - GROUP_TAIL_BYTES) / 2 & ~15u;
       const uint32_t want = (c.words * 4u + 15u) & ~15u;
